@@ -8,6 +8,8 @@
 // contiguous bytes; a transpose kernel produces the reference's pixel-major
 // [P, A] at the end.  The first pass writes without reading (the reference
 // resets the buffer to -inf before pass 0).
+#include <cmath>
+
 #include "march_core.cuh"
 
 namespace ls200 {
@@ -17,13 +19,14 @@ struct MarchParams {
     int azimuth_count, center_count, dem_count;
     const float *primary_cells;
     int primary_width, primary_height;
-    float primary_m6, primary_m9;
     const float *cells;   // sanitized level 0 + mips of the active DEM
     const float *bounds;  // four-cell bounds of those cells
     int width, height;
     int level_count;
     int4 levels[kMaxLevels];  // (cell offset, width, height, -)
-    float m6, m7, m9, m10, radius;
+    // Mean pixel size, column pixel size (m) and the primary's over the
+    // active DEM's column pixel size.
+    float resolution, column_res, ratio, radius;
     int tile_column, tile_row, tile_width, tile_height, subpatch, pass_index;
     float observer_elevation;
     float *slopes;  // [A, P]
@@ -41,17 +44,21 @@ struct SharedLevels {
     __device__ __forceinline__ int4 cells(int l) const { return t.cells[l]; }
 };
 
-// Resident 128-thread blocks per SM the register budget is sized for.  With
-// the f32x2 pairs and the Newton reciprocal, 9 (56 registers) marched 3.9 %
-// faster than 10 (48 registers, whose spills had grown) and 3.6 % faster than
-// 8 (64 registers) on site-scale tiles; 12 was slower.
+// Resident 128-thread blocks per SM the register budget is sized for.  The
+// settled steps (march_dem_far) issue 55 instructions each where the full
+// step took 137, and no pipe is full (FMA 59 %, issue slots 65-73 %): what
+// remains is latency, so the choice is between resident warps and spills.  A
+// site-scale tile (4096^2 at 5 m plus regional, 200 km, B200) takes 183 ms at
+// 7 (72 registers), 185 ms at 8 (64, a few spills), 198 ms at 9 and 218 ms at
+// 10; with the full step everywhere it took 298 ms, best at 9.
 #ifndef LS_MARCH_MIN_BLOCKS
-#define LS_MARCH_MIN_BLOCKS 9
+#define LS_MARCH_MIN_BLOCKS 7
 #endif
 // Adjacent pixels of one azimuth in a warp (a power of two up to 32); the
 // warp's other lanes take the next azimuths of the same pixels.  4 pixels x
-// 8 azimuths marched 4.3 % faster than 32 pixels x 1 azimuth on site-scale
-// tiles (8 px: 3.9 %, 16 px: 2.1 %), with the same results.
+// 8 azimuths marches the site-scale tile in 185 ms and the plain 512^2 tile in
+// 34.5 ms (2 px: 191 and 34.5, 8 px: 186 and 36.6, 16 px: 190 and 40.8), with
+// the same results.
 #ifndef LS_MARCH_LANES
 #define LS_MARCH_LANES 4
 #endif
@@ -67,21 +74,25 @@ static long long march_threads(int pixels, int azimuths) {
     return pixel_groups * azimuth_groups * 32;
 }
 
+// hypot_fused and mean_resolution on the host: fmaf, sqrtf and the sums round
+// as the device's, and the kernel then reads the result as a constant.
+static float host_hypot_fused(float a, float b) { return std::sqrt(std::fmaf(a, a, b * b)); }
+static float host_mean_resolution(float m6, float m7, float m9, float m10) {
+    return (host_hypot_fused(m6, m9) + host_hypot_fused(m7, m10)) * 0.5f;
+}
+
 template <bool kCount>
 __global__ void __launch_bounds__(128, LS_MARCH_MIN_BLOCKS)
     march_pass_kernel(const __grid_constant__ MarchParams P) {
     __shared__ LevelTable table;
-    const float column_res = hypot_fused(P.m6, P.m9);
-    const float resolution = mean_resolution(P.m6, P.m7, P.m9, P.m10);
     if (threadIdx.x < P.level_count)
-        fill_level(table, threadIdx.x, resolution, P.levels[threadIdx.x]);
+        fill_level(table, threadIdx.x, P.resolution, P.levels[threadIdx.x]);
     __syncthreads();
 
     const int pixel_count = P.tile_width * P.tile_height;
     const long long linear = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     int pixel, azimuth;
     if (kMarchLanes == 32) {
-        if (linear >= static_cast<long long>(pixel_count) * P.azimuth_count) return;
         pixel = static_cast<int>(linear % pixel_count);
         azimuth = static_cast<int>(linear / pixel_count);
     } else {
@@ -92,38 +103,43 @@ __global__ void __launch_bounds__(128, LS_MARCH_MIN_BLOCKS)
         const long long pixel_group = warp - azimuth_group * pixel_groups;
         pixel = static_cast<int>(pixel_group * kMarchLanes + lane % kMarchLanes);
         azimuth = static_cast<int>(azimuth_group * (32 / kMarchLanes) + lane / kMarchLanes);
-        if (pixel >= pixel_count || azimuth >= P.azimuth_count) return;
     }
+    const bool in_tile = pixel < pixel_count && azimuth < P.azimuth_count;
     const int row = pixel / P.tile_width;
     const int column = pixel % P.tile_width;
     float *out = P.slopes + static_cast<size_t>(azimuth) * pixel_count + pixel;
-    // Pixels outside the primary DEM keep the initial -inf sentinel.
-    if (P.tile_column + column >= P.primary_width || P.tile_row + row >= P.primary_height) {
-        if (P.first_pass) *out = -INFINITY;
-        return;
+    const bool marches = in_tile && P.tile_column + column < P.primary_width &&
+                         P.tile_row + row < P.primary_height;
+    RaySegment g{};
+    float observer_z = 0.0f, current = -1e30f;
+    if (marches) {
+        g = interpolate_segment(P.segments, P.center_count, P.dem_count, P.pass_index, azimuth,
+                                column, row, P.tile_column, P.tile_row, P.tile_width, P.subpatch,
+                                P.primary_width, P.primary_height, P.ratio);
+        observer_z = __fadd_rn(
+            bilinear(P.primary_cells, P.primary_width, P.primary_height,
+                     static_cast<float>(P.tile_column + column),
+                     static_cast<float>(P.tile_row + row)),
+            P.observer_elevation);
+        if (!P.first_pass) {
+            const float initial = *out;
+            current = isinf(initial) ? -1e30f : initial;
+        }
     }
-    const float ratio = __fdiv_rn(hypot_fused(P.primary_m6, P.primary_m9), column_res);
-    const RaySegment g = interpolate_segment(
-        P.segments, P.center_count, P.dem_count, P.pass_index, azimuth, column, row,
-        P.tile_column, P.tile_row, P.tile_width, P.subpatch, P.primary_width, P.primary_height,
-        ratio);
-    const float observer_z = __fadd_rn(
-        bilinear(P.primary_cells, P.primary_width, P.primary_height,
-                 static_cast<float>(P.tile_column + column),
-                 static_cast<float>(P.tile_row + row)),
-        P.observer_elevation);
-    float current = -1e30f;
-    if (!P.first_pass) {
-        const float initial = *out;
-        current = isinf(initial) ? -1e30f : initial;
-    }
-    const DemView dem{P.cells, P.bounds, P.width, P.height, P.level_count, resolution, column_res,
-                      P.radius};
+    const DemView dem{P.cells, P.bounds, P.width, P.height, P.level_count, P.resolution,
+                      P.column_res, P.radius};
+    __shared__ RayStore::Block store;
     unsigned visits = 0, samples = 0, steps = 0;
-    current = march_dem<kCount, kReference>(SharedLevels{table}, dem, g, P.pass_index, observer_z,
-                                       current, visits, samples, steps);
-    *out = current > -1e29f ? current : -INFINITY;
-    if (kCount) add_counters(P.counters, visits, samples, steps);
+    NoArgmax none;
+    current = march_dem_far<kCount, true>(SharedLevels{table}, dem, g, P.pass_index, observer_z,
+                                          current, marches, RayStore(store), visits, samples,
+                                          steps, none);
+    if (marches) {
+        *out = current > -1e29f ? current : -INFINITY;
+        if (kCount) add_counters(P.counters, visits, samples, steps);
+    } else if (in_tile && P.first_pass) {
+        *out = -INFINITY;  // pixels outside the primary DEM keep the sentinel
+    }
 }
 
 void march_pass_device(ls200_context *ctx, const MarchTile &tile, const ls200_dem *primary,
@@ -141,8 +157,6 @@ void march_pass_device(ls200_context *ctx, const MarchTile &tile, const ls200_de
     P.primary_cells = primary->cells;
     P.primary_width = primary->width;
     P.primary_height = primary->height;
-    P.primary_m6 = primary->map_parameters[6];
-    P.primary_m9 = primary->map_parameters[9];
     P.cells = active->cells;
     P.bounds = active->bounds;
     P.width = active->width;
@@ -152,10 +166,10 @@ void march_pass_device(ls200_context *ctx, const MarchTile &tile, const ls200_de
     for (int l = 0; l < active->level_count; ++l)
         P.levels[l] = make_int4(l == 0 ? 0 : cells0 + active->levels[l].offset,
                                 active->levels[l].width, active->levels[l].height, 0);
-    P.m6 = active->map_parameters[6];
-    P.m7 = active->map_parameters[7];
-    P.m9 = active->map_parameters[9];
-    P.m10 = active->map_parameters[10];
+    const float *m = active->map_parameters, *pm = primary->map_parameters;
+    P.resolution = host_mean_resolution(m[6], m[7], m[9], m[10]);
+    P.column_res = host_hypot_fused(m[6], m[9]);
+    P.ratio = host_hypot_fused(pm[6], pm[9]) / P.column_res;
     P.radius = static_cast<float>(active->projection[0]);
     P.tile_column = tile.tile_column;
     P.tile_row = tile.tile_row;

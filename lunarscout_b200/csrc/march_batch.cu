@@ -22,6 +22,7 @@
 #include "march_core.cuh"
 
 #include <map>
+#include <type_traits>
 #include <vector>
 
 namespace ls200 {
@@ -107,6 +108,7 @@ __global__ void __launch_bounds__(128, kMinBlocks)
     const int lanes = P.lanes_per_azimuth;
     const int azimuths_per_job = 32 / lanes;
     unsigned visits = 0, samples = 0, steps = 0;
+    __shared__ typename std::conditional<kLadder == kReference, RayStore::Block, char>::type store;
     for (;;) {
         unsigned long long taken = 0;
         if (lane == 0) taken = atomicAdd(P.next_job, 1ull);
@@ -118,7 +120,6 @@ __global__ void __launch_bounds__(128, kMinBlocks)
         const int pixel_group = static_cast<int>(local - azimuth_group * P.pixel_groups);
         const int pixel = pixel_group * lanes + lane % lanes;
         const int azimuth = azimuth_group * azimuths_per_job + lane / lanes;
-        if (azimuth >= P.azimuth_count) continue;
         const BatchTile &tile = P.tiles[t];
         const int row = pixel / kTileSide, column = pixel % kTileSide;
         const size_t ray = static_cast<size_t>(pixel) * P.azimuth_count + azimuth;
@@ -127,38 +128,48 @@ __global__ void __launch_bounds__(128, kMinBlocks)
         const int primary_width = primary.view.width, primary_height = primary.view.height;
         typename TrackerOf<kArgmax>::type tracker;
         const size_t checkpoint = static_cast<size_t>(t) * kTilePixels * P.azimuth_count + ray;
-        // Pixels outside the primary DEM keep the -inf sentinel.
-        if (tile.tile_column + column >= primary_width || tile.tile_row + row >= primary_height) {
-            *out = -INFINITY;
-            if (kArgmax) P.checkpoint_flags[checkpoint] = 0xff;
-            continue;
-        }
-        const float observer_z = __fadd_rn(
-            bilinear(primary.view.cells, primary_width, primary_height,
-                     static_cast<float>(tile.tile_column + column),
-                     static_cast<float>(tile.tile_row + row)),
-            tile.observer_elevation);
-        float current = -1e30f;
+        const bool in_tile = azimuth < P.azimuth_count;
+        const bool marches = in_tile && tile.tile_column + column < primary_width &&
+                             tile.tile_row + row < primary_height;
+        float observer_z = 0.0f, current = -1e30f;
+        if (marches)
+            observer_z = __fadd_rn(
+                bilinear(primary.view.cells, primary_width, primary_height,
+                         static_cast<float>(tile.tile_column + column),
+                         static_cast<float>(tile.tile_row + row)),
+                tile.observer_elevation);
         for (int d = 0; d < tile.dem_count; ++d) {
             const BatchDem &dem = P.dems[tile.dems[d]];
             const DemView view = dem.view;
-            const float ratio = __fdiv_rn(primary.view.column_res, view.column_res);
-            const RaySegment g = interpolate_segment<(kLadder & kRelative) != 0>(
-                tile.segments, P.center_count, tile.dem_count, d, azimuth, column, row,
-                tile.tile_column, tile.tile_row, kTileSide, P.subpatch, primary_width,
-                primary_height, ratio);
+            RaySegment g{};
+            if (marches) {
+                const float ratio = __fdiv_rn(primary.view.column_res, view.column_res);
+                g = interpolate_segment<(kLadder & kRelative) != 0>(
+                    tile.segments, P.center_count, tile.dem_count, d, azimuth, column, row,
+                    tile.tile_column, tile.tile_row, kTileSide, P.subpatch, primary_width,
+                    primary_height, ratio);
+            }
             if constexpr (kArgmax) tracker.current_pass = d;
-            current = march_dem_tracked<kCount, kLadder>(GlobalLevels{&dem.table}, view, g, d,
-                                                         observer_z, current, visits, samples,
-                                                         steps, tracker);
+            const GlobalLevels levels{&dem.table};
+            if constexpr (kLadder == kReference)
+                current = march_dem_far<kCount, false>(levels, view, g, d, observer_z, current,
+                                                       marches, RayStore(store), visits, samples,
+                                                       steps, tracker);
+            else if (marches)
+                current = march_dem_tracked<kCount, kLadder>(levels, view, g, d, observer_z,
+                                                             current, visits, samples, steps,
+                                                             tracker);
         }
+        if (!in_tile) continue;
         if constexpr (kArgmax) {
-            P.checkpoints[checkpoint] =
-                make_float4(tracker.px, tracker.py, tracker.true_m, tracker.slope);
+            if (marches)
+                P.checkpoints[checkpoint] =
+                    make_float4(tracker.px, tracker.py, tracker.true_m, tracker.slope);
             P.checkpoint_flags[checkpoint] =
                 tracker.pass < 0 ? uint8_t(0xff)
                                  : static_cast<uint8_t>((tracker.pass << 1) | tracker.near);
         }
+        // Pixels outside the primary DEM keep the -inf sentinel.
         float value = current > -1e29f ? current : -INFINITY;
         if (P.degrees && !isinf(value)) value = __fmul_rn(atanf(value), kSlopeDegrees);
         *out = value;

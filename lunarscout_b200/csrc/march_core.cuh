@@ -35,7 +35,10 @@
 //   * the tangent and its reciprocals depend only on the ray position and are
 //     computed once per position, not per level;
 //   * the cull test decides with a cheap bound outside a guard band and with
-//     the reference arithmetic inside it (bound_culled).
+//     the reference arithmetic inside it (bound_culled);
+//   * in the reference traversal most far-field culls are settled by a step
+//     of 55 instructions that computes exactly only what moves the ray
+//     (FarRay, march_dem_far), and most other steps by level0_step.
 //
 // The skip ladder (kLadder, the batched traversal; no reference counterpart)
 // extends a cull to the largest culled ancestor cell, see ladder_advance.
@@ -146,6 +149,20 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) {
     return d;
 }
 
+__device__ __forceinline__ float2 add2_down(float2 a, float2 b) {  // rounding down
+    float2 d;
+    asm("add.rm.f32x2 %0, %1, %2;"
+        : "=l"(reinterpret_cast<unsigned long long &>(d))
+        : "l"(reinterpret_cast<const unsigned long long &>(a)),
+          "l"(reinterpret_cast<const unsigned long long &>(b)));
+    return d;
+}
+__device__ __forceinline__ float sqrt_approx(float x) {
+    float y;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // The quartic path polynomial of both axes at once: lane x with
 // (start_x, a1..a4), lane y with (start_y, b1..b4); d2, d3, d4 are the powers
 // of the path offset d (cuda_backend.py:62-73).
@@ -158,11 +175,13 @@ __device__ __forceinline__ float2 quartic2(float2 x0, float2 k1, float2 k2, floa
     return __ffma2_rn(k4, d4, r);
 }
 
-// The Newton reciprocal of both lanes without the range fallback (the
-// caller handles |x| >= 2^64).
-__device__ __forceinline__ float2 newton_reciprocal_pair(float2 x) {
-    const float2 y = pair(rcp_approx(x.x), rcp_approx(x.y));
-    const float2 e = __ffma2_rn(__fmul2_rn(x, pair(-1.0f, -1.0f)), y, pair(1.0f, 1.0f));
+// The negated Newton reciprocal -1/x of both lanes without the range
+// fallback (the caller handles |x| >= 2^64).  Starting from y ~ 1/(-x) the
+// residual 1 - x/x is fma(x, y, 1) without negating x first, and every
+// rounding is that of the positive reciprocal with its sign turned.
+__device__ __forceinline__ float2 newton_minus_reciprocal_pair(float2 x) {
+    const float2 y = pair(rcp_approx(-x.x), rcp_approx(-x.y));
+    const float2 e = __ffma2_rn(x, y, pair(1.0f, 1.0f));
     return __ffma2_rn(y, e, y);
 }
 
@@ -170,7 +189,8 @@ __device__ __forceinline__ float2 newton_reciprocal_pair(float2 x) {
 // Newton step issued as f32x2 pairs; each lane needs |x| >= 2^-64.  The
 // march inlines the same choice with one branch for both lanes.
 __device__ __forceinline__ float2 reciprocal_pair(float2 x) {
-    float2 y = newton_reciprocal_pair(x);
+    float2 y = newton_minus_reciprocal_pair(x);
+    y = pair(-y.x, -y.y);
     if (!(fabsf(x.x) < 0x1p64f)) y.x = __frcp_rn(x.x);
     if (!(fabsf(x.y) < 0x1p64f)) y.y = __frcp_rn(x.y);
     return y;
@@ -385,15 +405,18 @@ __device__ __forceinline__ float cell_bound(const float *__restrict__ bounds, in
 // (bitwise the same value, including the -0.0 of a ray starting on the edge).
 // (ux, uy) is the position relative to the integer origin (origin_x,
 // origin_y); the reference arithmetic is origin 0 with u the absolute position.
+// minus_inv is the negated reciprocal of the tangent: (u - edge) * -1/t rounds
+// to the same value as (edge - u) * 1/t.
 __device__ __forceinline__ float cell_exit_advance(int shift, int cx, int cy, float ux, float uy,
-                                                   int origin_x, int origin_y, float inv_x,
-                                                   float inv_y, float fallback) {
+                                                   int origin_x, int origin_y,
+                                                   float2 minus_inv, float fallback) {
     const float scale_f = power_of_two(shift);
     const float2 low = pair(static_cast<float>((cx << shift) - origin_x),
                             static_cast<float>((cy << shift) - origin_y));
     const float2 high = __fadd2_rn(low, pair(scale_f, scale_f));
-    const float2 edge = pair(inv_x > 0.0f ? high.x : low.x, inv_y > 0.0f ? high.y : low.y);
-    const float2 tm = __fmul2_rn(sub2(edge, pair(ux, uy)), pair(inv_x, inv_y));
+    const float2 edge = pair(minus_inv.x < 0.0f ? high.x : low.x,
+                             minus_inv.y < 0.0f ? high.y : low.y);
+    const float2 tm = __fmul2_rn(sub2(pair(ux, uy), edge), minus_inv);
     const float tmx = tm.x, tmy = tm.y;
     const float exit_distance = tmx < tmy ? tmx : tmy;
     // The reference returns `fallback` when the distance it adds 1e-4 km to
@@ -427,16 +450,15 @@ __device__ __forceinline__ float cell_exit_advance(int shift, int cx, int cy, fl
 template <class Table>
 __device__ __forceinline__ bool ladder_culled(const Table &table, const float *__restrict__ bounds,
                                               int m, int ipx, int ipy, float ux, float uy,
-                                              int origin_x, int origin_y,
-                                              float inv_x, float inv_y, bool near, float true_m,
-                                              float radius, float observer_z,
+                                              int origin_x, int origin_y, float2 minus_inv,
+                                              bool near, float true_m, float radius, float observer_z,
                                               float observer_radius, float inverse_denominator,
                                               float current, float &step) {
     const int shift = 2 * m;
     const int cx = ipx >> shift, cy = ipy >> shift;
     const int4 L = table.cells(m);
     const float maximum_height = cell_bound(bounds, L, cx, cy);
-    step = cell_exit_advance(shift, cx, cy, ux, uy, origin_x, origin_y, inv_x, inv_y,
+    step = cell_exit_advance(shift, cx, cy, ux, uy, origin_x, origin_y, minus_inv,
                              __int_as_float(L.w));
     if (maximum_height < -20000.0f) return true;
     const float dh = __fsub_rn(maximum_height, observer_z);
@@ -479,8 +501,8 @@ template <bool kCount, class Table>
 __device__ __forceinline__ float ladder_advance(const Table &table, const float *__restrict__ bounds,
                                                 int level, int top, int ipx, int ipy, float ux,
                                                 float uy, int origin_x, int origin_y,
-                                                float inv_x, float inv_y, bool near,
-                                                float true_m, float radius, float observer_z,
+                                                float2 minus_inv, bool near, float true_m,
+                                                float radius, float observer_z,
                                                 float observer_radius, float inverse_denominator,
                                                 float current, float advance, unsigned &visits,
                                                 int &reached) {
@@ -490,7 +512,7 @@ __device__ __forceinline__ float ladder_advance(const Table &table, const float 
     for (int m = level + 1; m <= top; ++m) {
         float step;
         if (kCount) ++visits;
-        if (!ladder_culled(table, bounds, m, ipx, ipy, ux, uy, origin_x, origin_y, inv_x, inv_y,
+        if (!ladder_culled(table, bounds, m, ipx, ipy, ux, uy, origin_x, origin_y, minus_inv,
                            near, true_m, radius, observer_z, observer_radius,
                            inverse_denominator, current, step))
             break;
@@ -610,6 +632,7 @@ __device__ __forceinline__ MarchState begin_pass(const DemView &dem, const RaySe
 // (bit 0) and the relative arithmetic (bit 1).
 enum Traversal { kReference = 0, kLadderClimb = 1, kRelative = 2 };
 
+
 // Which level-0 sample set the running maximum: nothing (NoArgmax, the
 // production kernels) or its position, distance and slope (Argmax, the
 // checkpoint of the DEM adjoint; `pass` is set by the caller).
@@ -631,16 +654,414 @@ struct Argmax {
     }
 };
 
-// One outer iteration of hierarchy_maximum (cuda_backend.py:672-867): one ray
-// position, the level descent (and with the ladder the climb) and the advance.
-// Returns false, leaving `st` untouched, when the pass is over (past s_end,
-// outside the DEM, or the cell left the level grid).
+// Where a ray stands at path position s: DEM position p, the position u
+// relative to the integer origin (p itself in the reference arithmetic), the
+// tangent and its negated reciprocals, which depend on s alone.
+struct StepPoint {
+    float2 p, u;
+    float2 r;  // relative arithmetic: offset from the ray's start
+    float2 tangent, minus_inv;
+};
+
+template <bool kRelativeArithmetic>
+__device__ __forceinline__ StepPoint step_point(const RaySegment &g, float s) {
+    StepPoint at;
+    const float delta = __fsub_rn(s, g.s_start);
+    const float2 d1 = pair(delta, delta);
+    const float2 d2 = __fmul2_rn(d1, d1);
+    const float2 d3 = __fmul2_rn(d2, d1);
+    const float2 d4 = __fmul2_rn(d2, d2);
+    // Relative arithmetic: offsets along the ray without the start, added
+    // to the start relative to the origin; the absolute position (origin
+    // + offset, rounded) only takes the bounds decisions.
+    if (kRelativeArithmetic) {
+        at.r = quartic2(pair(0.0f, 0.0f), g.k1, g.k2, g.k3, g.k4, d1, d2, d3, d4);
+        at.u = __fadd2_rn(g.start, at.r);
+        at.p = __fadd2_rn(pair(static_cast<float>(g.origin_x), static_cast<float>(g.origin_y)),
+                          at.u);
+    } else {
+        at.p = quartic2(g.start, g.k1, g.k2, g.k3, g.k4, d1, d2, d3, d4);
+        at.u = at.p;
+    }
+    // The Newton reciprocal is exact for 2^-64 <= |d| < 2^64 and used only
+    // for |d| > 1e-8; march_step replaces the others.
+    at.tangent = quartic_tangent2(g.k1, g.k2, g.k3, g.k4, d1, d2, d3);
+    at.minus_inv = newton_minus_reciprocal_pair(at.tangent);
+    return at;
+}
+
+// Far-field culls settled without the reference's full step.
+//
+// Nine steps in ten of a ray are one culled visit beyond 500 m.  Such a step
+// needs exactly only what moves the ray (position, tangent reciprocals, cell
+// exit); the chord distance, the level and the bound's slope feed comparisons,
+// so a bound on their error may decide those.  With d the distance at the
+// cell's near side, dh = h - observer_z, E = 2 (R + observer_z) and sin the
+// sine of the running maximum's elevation, the reference's
+//   (dh (2R + h + observer_z) - d^2) / E / local_x <= current
+// is, local_x being sqrt(d^2 - local_z^2),
+//   dh (E + dh) <= d (d + E sin):
+// no division, no root.  The margins below cover every rounding of both
+// sides: the reference's slope is within 7e-7 (|dh| (E + |dh|) + d^2) / E of
+// its real value in local z; the approximate d within 2e-6 of the
+// reference's (8 roundings each, the chord's higher terms at most a fifth of
+// the linear one: see far_range), so with dn >= true_m / 2 the right side
+// moves by at most 4e-6 d (2d + E |sin|).
+//
+// The exit: the edges ahead are chosen by the signs of the tangent that the
+// last full step saw (`ahead`).  A wrong sign makes that axis' exit negative
+// or -0, and the step is not settled; +0 is a position on the edge itself,
+// which advances by the fallback.  A component within 1e-8 of zero, for which
+// the reference takes the reciprocal 1e30, is not settled either; at exactly
+// zero its exit is NaN, which the minimum drops as it would 1e30 pixels.
+//
+// A step that is not settled here (the bound too high or too close to tell,
+// another level, a wrong sign) goes to level0_step or the reference's step.
+// Half of the values sit in shared memory (RayStore) and are loaded at each
+// step: four 16-byte loads cost less than the resident warps that their
+// registers would.
+struct FarRay {
+    float end;            // s below which steps may settle (km; -inf: none)
+    float height_base;    // observer_z lowered by 5e-6 (32768 + |observer_z|)
+    float double_radius;  // E, raised by 4e-6
+    float sine;           // E sin, lowered by 8e-6; -inf when nothing culls
+};
+// Of the level of the previous step:
+struct FarLevel {
+    float chord_base;  // start chord (m) less the cell's side (m)
+    float low, high;   // dn range over which the level stays the reference's
+    float fallback;    // the level's advance when no edge lies ahead (km)
+};
+struct FarCell {
+    float rounder;       // 2^23 4^level: adding it rounds down to a cell edge
+    float2 ahead;        // 4^level - rounder where the tangent rises, else -rounder
+    unsigned row, base;  // index = bits(rounded y) * row + bits(rounded x) + base
+};
+
+// Per-ray values outside the registers, one column per thread of a 128-thread
+// block.  Volatile accesses: the compiler must not carry them in registers.
+struct RayStore {
+    static constexpr int kQuads = 2;
+    enum Field { kCurrent, kSideUp, kSideHere, kLevel, kEnd, kChord, kObserver, kLimit, kFields };
+    struct Block {
+        float4 quads[kQuads][128];
+        float fields[kFields][128];
+    };
+    unsigned quad;           // shared address of the thread's first quad
+    volatile float *column;  // the thread's first field
+    __device__ __forceinline__ explicit RayStore(Block &block)
+        : quad(static_cast<unsigned>(__cvta_generic_to_shared(&block.quads[0][threadIdx.x]))),
+          column(&block.fields[0][threadIdx.x]) {}
+    __device__ __forceinline__ float get(Field f) const { return column[f * 128]; }
+    __device__ __forceinline__ void set(Field f, float v) const { column[f * 128] = v; }
+    __device__ __forceinline__ float4 load(int i) const {
+        float4 v;
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                     : "r"(quad + i * 2048u) : "memory");
+        return v;
+    }
+    __device__ __forceinline__ void save(int i, float x, float y, float z, float w) const {
+        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};"
+                     :: "r"(quad + i * 2048u), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+    }
+    __device__ __forceinline__ FarRay ray() const {
+        const float4 v = load(0);
+        return FarRay{v.x, v.y, v.z, v.w};
+    }
+    __device__ __forceinline__ FarLevel level() const {
+        const float4 v = load(1);
+        return FarLevel{v.x, v.y, v.z, v.w};
+    }
+};
+
+__device__ __forceinline__ float far_sine(float observer_radius, float current) {
+    const float slope = fminf(current, 1e4f);
+    const float scaled = 2.0f * observer_radius * (slope * rsqrtf(1.0f + slope * slope));
+    // Nothing settles before the first sample.  A steep maximum needs no
+    // limit: with the sine lowered by 8e-6 the slopes that settle stay below
+    // 400, where local_x^2 is still 20 times its rounding.
+    return current >= -30.0f ? scaled - 8e-6f * fabsf(scaled) : -INFINITY;
+}
+
+// The values of `level`, and the edges ahead for a tangent.
+template <class Table>
+__device__ __forceinline__ void far_level(FarCell &far, const RayStore &store, const Table &table,
+                                          const DemView &dem, float start_chord_km, int level) {
+    const int4 cells = table.cells(level);
+    far.rounder = power_of_two(2 * level + 23);
+    const unsigned bits = __float_as_uint(far.rounder);
+    far.row = static_cast<unsigned>(cells.y);
+    far.base = static_cast<unsigned>(cells.x) - bits * (far.row + 1u);
+    const float side = power_of_two(2 * level) * dem.resolution;
+    // side <= footprint(true_m) < side above, footprint = true_m * 0.25 deg.
+    constexpr float kReach = 229.1831180523293f;
+    const float least = level > 0 ? table.side(level) * kReach * 1.00001f : 0.0f;
+    store.save(1, start_chord_km * 1000.0f - side, fmaxf(least, 2.0f * side + 2.0f) - side,
+               level < dem.level_count - 1 ? table.side(level + 1) * kReach * 0.99999f - side
+                                           : INFINITY,
+               __int_as_float(cells.w));
+}
+
+__device__ __forceinline__ void far_ahead(FarCell &far, float2 tangent) {
+    const float cell = far.rounder * 0x1p-23f;
+    far.ahead = pair((tangent.x < -1e-8f ? 0.0f : cell) - far.rounder,
+                     (tangent.y < -1e-8f ? 0.0f : cell) - far.rounder);
+}
+
+// The s range in which steps may settle.  The segment must keep the
+// approximations' error bounds (finite, of ordinary size, the chord
+// polynomial's higher terms within a fifth of its linear one, the path
+// bounded by its coefficients), the DEM must be small enough for exact float
+// cell edges, and the path must stay inside the DEM by more than its
+// rounding: the Bernstein coefficients of the quartic over the range enclose
+// it.  A segment usually ends at the DEM's edge, so the range stops 1/256
+// short of it, or 1/16 where the path leaves at a shallow angle; a path that
+// hugs an edge gets an empty range.
+struct FarRange {
+    bool tame;  // the error bounds hold on the whole segment
+    float end;  // steps may settle from 500 m up to here (km; -inf: none)
+};
+
+__device__ __forceinline__ FarRange far_range(const DemView &dem, const RaySegment &g,
+                                              float observer_z) {
+    const float span = g.s_end - g.s_start;
+    const float reach =
+        span * (fabsf(g.k1.x) + fabsf(g.k1.y) +
+                span * (fabsf(g.k2.x) + fabsf(g.k2.y) +
+                        span * (fabsf(g.k3.x) + fabsf(g.k3.y) +
+                                span * (fabsf(g.k4.x) + fabsf(g.k4.y)))));
+    const float planar = reach * dem.resolution * 1.0001f;
+    const bool tame = span >= 1e-3f && reach < 4e6f && fabsf(g.start.x) < 4e6f &&
+                      fabsf(g.start.y) < 4e6f && g.s_start_chord >= 0.0f &&
+                      g.s_start_chord < 1e6f && g.c1 >= 0.1f && g.c1 <= 10.0f &&
+                      planar * (fabsf(g.c2) + planar * fabsf(g.c3)) <= 0.2f * g.c1 &&
+                      dem.width <= (1 << 22) && dem.height <= (1 << 22) &&
+                      fabsf(observer_z) < 1e6f && dem.radius > 1e5f && dem.radius < 1e9f;
+    const float a = fmaxf(0.5f - g.s_start, 0.0f);
+    const float2 a2 = pair(a, a);
+    const float2 t0 = __ffma2_rn(a2, __ffma2_rn(a2, __ffma2_rn(a2, __ffma2_rn(a2, g.k4, g.k3),
+                                                               g.k2), g.k1), g.start);
+    // Derivatives at `a` over 1!, 2! and 3!.
+    const float2 p3 = __fmul2_rn(pair(3.0f, 3.0f), g.k3), p4 = __fmul2_rn(a2, g.k4);
+    const float2 d1 = __ffma2_rn(a2, __ffma2_rn(a2, __ffma2_rn(pair(4.0f, 4.0f), p4, p3),
+                                                __fadd2_rn(g.k2, g.k2)), g.k1);
+    const float2 d2 = __ffma2_rn(a2, __ffma2_rn(pair(6.0f, 6.0f), p4, p3), g.k2);
+    const float2 d3 = __ffma2_rn(pair(4.0f, 4.0f), p4, g.k3);
+    const float margin = 1.0f + 1e-5f * (reach + fabsf(g.start.x) + fabsf(g.start.y));
+    FarRange range{tame, -INFINITY};
+    if (!tame) return range;
+    for (float part = 0.00390625f; part < 0.5f; part *= 16.0f) {
+        const float w = (span - a) * (1.0f - part);
+        if (!(w > 0.0f)) break;
+        const float2 w2 = pair(w, w), w3 = pair(w * w, w * w);
+        const float2 t1 = __fmul2_rn(w2, d1), t2 = __fmul2_rn(w3, d2);
+        const float2 t3 = __fmul2_rn(__fmul2_rn(w3, w2), d3);
+        const float2 t4 = __fmul2_rn(__fmul2_rn(w3, w3), g.k4);
+        const float2 b1 = __ffma2_rn(pair(0.25f, 0.25f), t1, t0);
+        const float2 b2 = __ffma2_rn(pair(1.0f / 6, 1.0f / 6), t2,
+                                     __ffma2_rn(pair(0.5f, 0.5f), t1, t0));
+        const float2 b3 = __ffma2_rn(pair(0.25f, 0.25f), t3,
+                                     __ffma2_rn(pair(0.5f, 0.5f), t2,
+                                                __ffma2_rn(pair(0.75f, 0.75f), t1, t0)));
+        const float2 b4 = __fadd2_rn(__fadd2_rn(__fadd2_rn(t0, t1), __fadd2_rn(t2, t3)), t4);
+        const float least_x = fminf(fminf(fminf(t0.x, b1.x), fminf(b2.x, b3.x)), b4.x);
+        const float least_y = fminf(fminf(fminf(t0.y, b1.y), fminf(b2.y, b3.y)), b4.y);
+        const float most_x = fmaxf(fmaxf(fmaxf(t0.x, b1.x), fmaxf(b2.x, b3.x)), b4.x);
+        const float most_y = fmaxf(fmaxf(fmaxf(t0.y, b1.y), fmaxf(b2.y, b3.y)), b4.y);
+        if (least_x > margin && least_y > margin &&
+            most_x < static_cast<float>(dem.width - 1) - margin &&
+            most_y < static_cast<float>(dem.height - 1) - margin) {
+            range.end = fminf(g.s_start + a + w, g.s_end);
+            break;
+        }
+    }
+    return range;
+}
+
+// The step from path position `s` at DEM position `p`: true when it is a
+// cull that could be settled; `s` then is the next path position.
+__device__ __forceinline__ bool far_step(const FarCell &far, const RayStore &store,
+                                         const DemView &dem, const RaySegment &g, float2 p,
+                                         float2 minus_inv, float &s) {
+    const FarRay ray = store.ray();
+    const bool in = s < ray.end;
+    const float2 down = add2_down(p, pair(far.rounder, far.rounder));
+    const unsigned index =
+        __float_as_uint(down.y) * far.row + __float_as_uint(down.x) + far.base;
+    float height = INFINITY;  // settles nothing
+    if (in) height = __ldg(dem.bounds + static_cast<int>(index));
+    const FarLevel at = store.level();
+    const float2 r = sub2(p, g.start);
+    const float planar = sqrt_approx(__fmaf_rn(r.x, r.x, r.y * r.y)) * dem.resolution;
+    const float dn = __fmaf_rn(
+        planar, __fmaf_rn(planar, __fmaf_rn(planar, g.c3, g.c2), g.c1), at.chord_base);
+    // down + (4^level - rounder) and down - rounder are exact.
+    const float2 exits = __fmul2_rn(sub2(p, __fadd2_rn(down, far.ahead)), minus_inv);
+    const float exit = fminf(exits.x, exits.y);
+    const float dh = height - ray.height_base;
+    const float left = dh * (dh + ray.double_radius);
+    const float right = dn * __fmaf_rn(dn, 0.999988f, ray.sine);
+    const float next = __fadd_rn(s, __fadd_rn(exit > 0.0f ? exit : at.fallback, 0.0001f));
+    const bool settled = left < right && dn > at.low && dn < at.high &&
+                         __float_as_int(exit) >= 0 &&
+                         fmaxf(fabsf(minus_inv.x), fabsf(minus_inv.y)) < 9e7f;
+    if (settled) s = next;
+    return settled;
+}
+
+// x / 1000 correctly rounded (for normal x and quotient): a faithful quotient
+// corrected by its exact residual (Markstein, as rcp_approx); equal to the
+// IEEE division for every significand.
+__device__ __forceinline__ float over_1000(float x) {
+    const float q = __fmul_rn(x, 0.001f);
+    return __fmaf_rn(__fmaf_rn(-1000.0f, q, x), 0.001f, q);
+}
+
+// The chord distance of a far-field position in the reference's rounding.
+__device__ __forceinline__ float chord_distance_m(const RaySegment &g, float2 r,
+                                                  float resolution) {
+    const float2 planar = __fmul2_rn(r, pair(resolution, resolution));
+    const float planar_m = hypot_fused(planar.x, planar.y);
+    const float pm2 = __fmul_rn(planar_m, planar_m);
+    // (c2 * pm2, pm2 * planar_m) in one instruction.
+    const float2 terms = __fmul2_rn(pair(g.c2, pm2), pair(pm2, planar_m));
+    float chord = __fmaf_rn(g.c1, planar_m, terms.x);
+    chord = __fmaf_rn(g.c3, terms.y, chord);
+    return __fmaf_rn(g.s_start_chord, 1000.0f, chord);
+}
+
+// One step at level 0 in the reference's arithmetic, for the rays far_range
+// found tame and positions whose clamps do not act: most steps that far_step
+// leaves over, in the near field all.  Returns false, having done nothing,
+// when the step is another one.  The cull (one product per side) and which
+// of pixel, angular and floor step is the largest are again decided by a
+// bound on the error where that is clear.
+template <bool kCount, bool kAhead, class Table, class Tracker>
+__device__ __forceinline__ bool level0_step(const Table &table, const DemView &dem,
+                                            const RaySegment &g, const StepPoint &at,
+                                            int pass_index, float observer_z, MarchState &st,
+                                            unsigned &samples, Tracker &tracker) {
+    const float2 p = at.p, tangent = at.tangent, minus_inv = at.minus_inv;
+    const float s = st.s, current = st.current;
+    const float resolution = dem.resolution;
+    const float xmax = fminf(static_cast<float>(dem.width) - 1.0001f,
+                             static_cast<float>(dem.width - 1) - 0.5f);
+    const float ymax = fminf(static_cast<float>(dem.height) - 1.0001f,
+                             static_cast<float>(dem.height - 1) - 0.5f);
+    if (!(st.level_hint == 0 && p.x >= 0.0f && p.y >= 0.0f && p.x < xmax &&
+          p.y < ymax && fabsf(tangent.x) > 1e-8f && fabsf(tangent.y) > 1e-8f))
+        return false;
+    const bool near = s < 0.5f;
+    const float true_m =
+        near ? __fmul_rn(s, 1000.0f) : chord_distance_m(g, sub2(p, g.start), resolution);
+    if (st.side_up <= __fmul_rn(true_m, 0.004363323129985824f)) return false;
+    const float2 down = add2_down(p, pair(0x1p23f, 0x1p23f));
+    const float2 corner = __fadd2_rn(down, pair(-0x1p23f, -0x1p23f));
+    const int index = (__float_as_int(down.y) - 0x4b000000) * dem.width +
+                      (__float_as_int(down.x) - 0x4b000000);
+    // kAhead: the corners are loaded along with the bound, before it is known
+    // whether they are needed: one memory latency per step instead of two.
+    const float *r0 = dem.cells + index, *r1 = r0 + dem.width;
+    float q00, q10, q01, q11;
+    if (kAhead) {
+        q00 = __ldg(r0), q10 = __ldg(r0 + 1);
+        q01 = __ldg(r1), q11 = __ldg(r1 + 1);
+    }
+    const float maximum_height = __ldg(dem.bounds + index);
+    const float observer_radius = __fadd_rn(dem.radius, observer_z);
+    const float denominator = __fmul_rn(2.0f, observer_radius);
+    bool culled = maximum_height < -20000.0f;
+    if (!culled) {
+        float true_near = __fsub_rn(true_m, resolution);
+        true_near = true_near > 1.0f ? true_near : 1.0f;
+        const float dh = __fsub_rn(maximum_height, observer_z);
+        float left, right, band;
+        if (near) {
+            left = dh;
+            right = current * true_near;
+            band = 1e-5f * fabsf(right) + 1e-30f;
+        } else {
+            const float sine = denominator * (current * rsqrtf(1.0f + current * current));
+            left = dh * (denominator + dh);
+            right = true_near * (true_near + sine);
+            band = 2e-5f * (fabsf(left) + true_near * (true_near + fabsf(sine)));
+            if (!(fabsf(current) <= 30.0f)) band = INFINITY;
+        }
+        culled = left < right - band;
+        if (!culled && !(left > right + band)) {
+            const float possible =
+                near ? __fdiv_rn(dh, true_near)
+                     : bound_slope(true_near, maximum_height, dem.radius, observer_z,
+                                   observer_radius);
+            culled = possible <= current;
+        }
+    }
+    if (culled) {
+        const float2 edge = __fadd2_rn(corner, pair(tangent.x > 0.0f ? 1.0f : 0.0f,
+                                                    tangent.y > 0.0f ? 1.0f : 0.0f));
+        const float2 exits = __fmul2_rn(sub2(p, edge), minus_inv);
+        const float exit = fminf(exits.x, exits.y);
+        st.s = __fadd_rn(s, __fadd_rn(exit > 0.0f ? exit : table.fallback(0), 0.0001f));
+        return true;
+    }
+    if (kCount) ++samples;
+    if (!kAhead) {
+        q00 = __ldg(r0), q10 = __ldg(r0 + 1);
+        q01 = __ldg(r1), q11 = __ldg(r1 + 1);
+    }
+    const bool valid = q00 > -20000.0f && q10 > -20000.0f && q01 > -20000.0f && q11 > -20000.0f;
+    const float2 t = sub2(p, corner);
+    const float top = __fmaf_rn(t.x, __fsub_rn(q10, q00), q00);
+    const float bottom = __fmaf_rn(t.x, __fsub_rn(q11, q01), q01);
+    const float height = __fmaf_rn(t.y, __fsub_rn(bottom, top), top);
+    float slope = -1e30f;
+    if (valid) {
+        slope = near ? __fdiv_rn(__fsub_rn(height, observer_z), true_m)
+                     : sample_slope(true_m, height, dem.radius, observer_radius);
+        if (slope > current) {
+            st.current = slope;
+            tracker.record(p.x, p.y, true_m, slope, near);
+        }
+    }
+    // The smaller of the margin's and the angular product, over 1000 (see
+    // march_step).
+    const float angular = __fmul_rn(true_m, 0.00151f);
+    const float margin = __fsub_rn(st.current, slope);
+    float product = 0.0f;
+    if (margin > 0.0f) {
+        const float margin_product = __fmul_rn(__fmul_rn(margin, true_m), 1.732f);
+        product = margin_product < angular ? margin_product : angular;
+    }
+    const float floor_step = pass_index == 0 && true_m >= 100.0f
+                                 ? __fmul_rn(__fmul_rn(0.8f, resolution), 0.001f)
+                                 : __fmul_rn(__fmul_rn(0.5f, resolution), 0.001f);
+    const float scale = near ? 0.25f : 1.0f;
+    float advance = over_1000(product);
+    const float squared = tangent.x * tangent.x + tangent.y * tangent.y;
+    const float pixel_most = rsqrtf(squared) * 1.00001f;
+    if (!(squared > 1e-11f) ||
+        !(advance > pixel_most || pixel_most * scale < floor_step * 0.99999f)) {
+        const float magnitude = hypot_fused(tangent.x, tangent.y);
+        const float pixel_step = magnitude > 1e-6f ? __frcp_rn(magnitude) : 0.0005f;
+        advance = pixel_step > advance ? pixel_step : advance;
+    }
+    advance = __fmul_rn(advance, scale);
+    advance = advance > floor_step ? advance : floor_step;
+    st.s = __fadd_rn(s, advance);
+    return true;
+}
+
+// One outer iteration of hierarchy_maximum (cuda_backend.py:672-867) at a
+// position s <= s_end: the level descent (and with the ladder the climb) and
+// the advance.  Returns false, leaving `st` untouched, when the pass is over
+// (outside the DEM, or the cell left the level grid).
 template <bool kCount, int kLadder, class Table, class Tracker>
-__device__ __forceinline__ bool march_step_tracked(const Table &table, const DemView &dem,
-                                                   const RaySegment &g, int pass_index,
-                                                   float observer_z, MarchState &st,
-                                                   unsigned &visits, unsigned &samples,
-                                                   unsigned &steps, Tracker &tracker) {
+__device__ __forceinline__ bool march_step(const Table &table, const DemView &dem,
+                                           const RaySegment &g, const StepPoint &at,
+                                           int pass_index, float observer_z, MarchState &st,
+                                           unsigned &visits, unsigned &samples,
+                                           unsigned &steps, Tracker &tracker) {
     const float radius = dem.radius;
     const float resolution = dem.resolution;
     const float observer_radius = __fadd_rn(radius, observer_z);
@@ -656,26 +1077,17 @@ __device__ __forceinline__ bool march_step_tracked(const Table &table, const Dem
     int level_hint = st.level_hint;
     float side_up = st.side_up, side_here = st.side_here;
     constexpr bool relative = (kLadder & kRelative) != 0;
-    if (!(s <= g.s_end)) return false;
     {
         if (kCount) ++steps;
-        const float delta = __fsub_rn(s, g.s_start);
-        const float2 d1 = pair(delta, delta);
-        const float2 d2 = __fmul2_rn(d1, d1);
-        const float2 d3 = __fmul2_rn(d2, d1);
-        const float2 d4 = __fmul2_rn(d2, d2);
-        // Relative arithmetic: offsets along the ray without the start, added
-        // to the start relative to the origin; the absolute position (origin
-        // + offset, rounded) only takes the bounds decisions.
-        float2 r, u, p;
-        if (relative) {
-            r = quartic2(pair(0.0f, 0.0f), g.k1, g.k2, g.k3, g.k4, d1, d2, d3, d4);
-            u = __fadd2_rn(g.start, r);
-            p = __fadd2_rn(pair(static_cast<float>(g.origin_x), static_cast<float>(g.origin_y)),
-                           u);
-        } else {
-            p = quartic2(g.start, g.k1, g.k2, g.k3, g.k4, d1, d2, d3, d4);
-            u = p;
+        const float2 u = at.u, p = at.p;
+        const float dx = at.tangent.x, dy = at.tangent.y;
+        float2 minus_inv = at.minus_inv;
+        const float ax = fabsf(dx), ay = fabsf(dy);
+        if (!(ax > 1e-8f)) minus_inv.x = -1e30f;
+        if (!(ay > 1e-8f)) minus_inv.y = -1e30f;
+        if (!(ax < 0x1p64f && ay < 0x1p64f)) {
+            minus_inv.x = ax > 1e-8f ? -__frcp_rn(dx) : -1e30f;
+            minus_inv.y = ay > 1e-8f ? -__frcp_rn(dy) : -1e30f;
         }
         const float ux = u.x, uy = u.y, px = p.x, py = p.y;
         // NaN fails every comparison, as the reference's isnan tests do.
@@ -686,15 +1098,7 @@ __device__ __forceinline__ bool march_step_tracked(const Table &table, const Dem
             true_m = __fmul_rn(s, 1000.0f);
         } else {
             // The planar distance only feeds the far-field chord.
-            if (!relative) r = sub2(p, g.start);
-            const float2 planar = __fmul2_rn(r, pair(resolution, resolution));
-            const float planar_m = hypot_fused(planar.x, planar.y);
-            const float pm2 = __fmul_rn(planar_m, planar_m);
-            // (c2 * pm2, pm2 * planar_m) in one instruction.
-            const float2 terms = __fmul2_rn(pair(g.c2, pm2), pair(pm2, planar_m));
-            float chord = __fmaf_rn(g.c1, planar_m, terms.x);
-            chord = __fmaf_rn(g.c3, terms.y, chord);
-            true_m = __fmaf_rn(g.s_start_chord, 1000.0f, chord);
+            true_m = chord_distance_m(g, relative ? at.r : sub2(p, g.start), resolution);
         }
         const float footprint = __fmul_rn(true_m, 0.004363323129985824f);
         // The reference scans down from the top level to the largest level
@@ -710,20 +1114,6 @@ __device__ __forceinline__ bool march_step_tracked(const Table &table, const Dem
             level_hint = level;
             side_up = level < top_level ? table.side(level + 1) : __int_as_float(0x7fffffff);
             side_here = level > 0 ? table.side(level) : -INFINITY;
-        }
-        // The tangent and its reciprocals depend only on delta.
-        const float2 tangent = quartic_tangent2(g.k1, g.k2, g.k3, g.k4, d1, d2, d3);
-        const float dx = tangent.x, dy = tangent.y;
-        // The Newton reciprocal is exact for 2^-64 <= |d| < 2^64 and used only
-        // for |d| > 1e-8; a tangent of 2^64 or more (or not finite) takes the
-        // IEEE reciprocal on a branch of its own.
-        const float2 newton = newton_reciprocal_pair(tangent);
-        const float ax = fabsf(dx), ay = fabsf(dy);
-        float inv_x = ax > 1e-8f ? newton.x : 1e30f;
-        float inv_y = ay > 1e-8f ? newton.y : 1e30f;
-        if (!(ax < 0x1p64f && ay < 0x1p64f)) {
-            inv_x = ax > 1e-8f ? __frcp_rn(dx) : 1e30f;
-            inv_y = ay > 1e-8f ? __frcp_rn(dy) : 1e30f;
         }
         const int origin_x = relative ? g.origin_x : 0;
         const int origin_y = relative ? g.origin_y : 0;
@@ -741,8 +1131,8 @@ __device__ __forceinline__ bool march_step_tracked(const Table &table, const Dem
                 break;
             }
             const float maximum_height = cell_bound(dem.bounds, L, cx, cy);
-            const float skip = cell_exit_advance(shift, cx, cy, ux, uy, origin_x, origin_y, inv_x,
-                                                 inv_y, __int_as_float(L.w));
+            const float skip = cell_exit_advance(shift, cx, cy, ux, uy, origin_x, origin_y, minus_inv,
+                                                 __int_as_float(L.w));
             bool culled = maximum_height < -20000.0f;
             if (!culled) {
                 const float scale_f = power_of_two(shift);
@@ -756,7 +1146,7 @@ __device__ __forceinline__ bool march_step_tracked(const Table &table, const Dem
                 if (kLadder & kLadderClimb) {
                     int reached;
                     advance = ladder_advance<kCount>(table, dem.bounds, level, top_level, ipx, ipy,
-                                                     ux, uy, origin_x, origin_y, inv_x, inv_y,
+                                                     ux, uy, origin_x, origin_y, minus_inv,
                                                      near, true_m, radius, observer_z,
                                                      observer_radius, inverse_denominator,
                                                      current, skip, visits, reached);
@@ -829,16 +1219,6 @@ __device__ __forceinline__ bool march_step_tracked(const Table &table, const Dem
 // hierarchy_maximum (cuda_backend.py:656-874): the maximum slope along one
 // ray over one DEM, starting from `current` (-1e30 for none).  Table gives
 // side(l), fallback(l), out_step(l) and cells(l).
-template <bool kCount, int kLadder, class Table>
-__device__ __forceinline__ bool march_step(const Table &table, const DemView &dem,
-                                           const RaySegment &g, int pass_index,
-                                           float observer_z, MarchState &st, unsigned &visits,
-                                           unsigned &samples, unsigned &steps) {
-    NoArgmax none;
-    return march_step_tracked<kCount, kLadder>(table, dem, g, pass_index, observer_z, st,
-                                               visits, samples, steps, none);
-}
-
 template <bool kCount, int kLadder, class Table, class Tracker>
 __device__ __forceinline__ float march_dem_tracked(const Table &table, const DemView &dem,
                                                    const RaySegment &g, int pass_index,
@@ -846,20 +1226,118 @@ __device__ __forceinline__ float march_dem_tracked(const Table &table, const Dem
                                                    unsigned &visits, unsigned &samples,
                                                    unsigned &steps, Tracker &tracker) {
     MarchState st = begin_pass(dem, g, current);
-    while (march_step_tracked<kCount, kLadder>(table, dem, g, pass_index, observer_z, st,
-                                               visits, samples, steps, tracker)) {
+    while (st.s <= g.s_end &&
+           march_step<kCount, kLadder>(table, dem, g,
+                                       step_point<(kLadder & kRelative) != 0>(g, st.s),
+                                       pass_index, observer_z, st, visits, samples, steps,
+                                       tracker)) {
     }
     return st.current;
 }
 
-template <bool kCount, int kLadder, class Table>
-__device__ __forceinline__ float march_dem(const Table &table, const DemView &dem,
-                                           const RaySegment &g, int pass_index,
-                                           float observer_z, float current, unsigned &visits,
-                                           unsigned &samples, unsigned &steps) {
-    NoArgmax none;
-    return march_dem_tracked<kCount, kLadder>(table, dem, g, pass_index, observer_z, current,
-                                              visits, samples, steps, none);
+// The step of a lane that far_step left over: level0_step or the reference's
+// full step, and what they change for the next fast steps.
+template <bool kCount, bool kAhead, class Table, class Tracker>
+__device__ __forceinline__ void slow_step(FarCell &far, const RayStore &store, const Table &table,
+                                          const DemView &dem, const RaySegment &g,
+                                          const StepPoint &at, int pass_index, float s_end,
+                                          float &s, unsigned &visits, unsigned &samples,
+                                          unsigned &steps, Tracker &tracker) {
+    RaySegment own = g;
+    own.s_end = s_end;
+    own.s_start_chord = store.get(RayStore::kChord);
+    const float z = store.get(RayStore::kObserver);
+    const float limit = store.get(RayStore::kLimit);
+    const float before = store.get(RayStore::kCurrent);
+    const int level = __float_as_int(store.get(RayStore::kLevel));
+    MarchState st{s, before, level, store.get(RayStore::kSideUp),
+                  store.get(RayStore::kSideHere)};
+    bool alive = true;
+    if (limit < INFINITY &&
+        level0_step<kCount, kAhead>(table, dem, own, at, pass_index, z, st, samples, tracker)) {
+        if (kCount) ++steps, ++visits;
+    } else {
+        alive = march_step<kCount, kReference>(table, dem, own, at, pass_index, z, st, visits,
+                                               samples, steps, tracker);
+    }
+    if (st.level_hint != level) {
+        far_level(far, store, table, dem, own.s_start_chord, st.level_hint);
+        store.set(RayStore::kLevel, __int_as_float(st.level_hint));
+        store.set(RayStore::kSideUp, st.side_up);
+        store.set(RayStore::kSideHere, st.side_here);
+    }
+    far_ahead(far, at.tangent);
+    s = alive ? st.s : INFINITY;
+    FarRay ray = store.ray();
+    ray.end = s >= 0.5f && limit < INFINITY ? limit : -INFINITY;
+    if (st.current != before) {
+        ray.sine = far_sine(dem.radius + z, st.current);
+        store.set(RayStore::kCurrent, st.current);
+    }
+    store.save(0, ray.end, ray.height_base, ray.double_radius, ray.sine);
+}
+
+// The reference traversal with its far-field culls settled by far_step.
+// Every lane of the warp calls it; `marches` is false for a lane without a
+// ray.  The fast step has no branch; the lanes it leaves over step together.
+// The votes also keep the warp together: without one per step the settled
+// lanes ran ahead while the others waited (4.3 times slower).
+// kNearFirst marches the near field, where no step settles, in a loop of its
+// own and loads corners ahead, which shortens a launch of few warps (the
+// 16 x 16 x 72 ray preview 282 -> 265 us, the site-scale tile 185.3 -> 183.3
+// ms); the persistent kernel, already out of registers, does without (212
+// instead of 221 ms on two sites).
+template <bool kCount, bool kNearFirst, class Table, class Tracker>
+__device__ __forceinline__ float march_dem_far(const Table &table, const DemView &dem,
+                                               const RaySegment &g, int pass_index,
+                                               float observer_z, float current, bool marches,
+                                               const RayStore &store, unsigned &visits,
+                                               unsigned &samples, unsigned &steps,
+                                               Tracker &tracker) {
+    const MarchState first = begin_pass(dem, g, current);
+    const FarRange range = far_range(dem, g, observer_z);
+    // A lane whose ray has ended (or never was) stands at +inf.
+    float s = marches ? first.s : INFINITY;
+    const float height_base = observer_z - 5e-6f * (32768.0f + fabsf(observer_z));
+    const float double_radius = 2.0f * (dem.radius + observer_z) * 1.000004f;
+    FarCell far;
+    far_level(far, store, table, dem, g.s_start_chord, first.level_hint);
+    far_ahead(far, pair(-1.0f, -1.0f));
+    store.save(0, s >= 0.5f ? range.end : -INFINITY, height_base, double_radius,
+               far_sine(dem.radius + observer_z, current));
+    store.set(RayStore::kCurrent, first.current);
+    store.set(RayStore::kSideUp, first.side_up);
+    store.set(RayStore::kSideHere, first.side_here);
+    store.set(RayStore::kLevel, __int_as_float(first.level_hint));
+    store.set(RayStore::kEnd, g.s_end);
+    store.set(RayStore::kChord, g.s_start_chord);
+    store.set(RayStore::kObserver, observer_z);
+    store.set(RayStore::kLimit, range.tame ? range.end : INFINITY);  // +inf: not tame
+    // The near field: every step is a full one.
+    bool near = kNearFirst && s < 0.5f;
+    while (kNearFirst && __any_sync(0xffffffffu, near)) {
+        const float s_end = store.get(RayStore::kEnd);
+        if (near && !(s <= s_end)) s = INFINITY;
+        else if (near) {
+            const StepPoint at = step_point<false>(g, s);
+            slow_step<kCount, true>(far, store, table, dem, g, at, pass_index, s_end, s,
+                                    visits, samples, steps, tracker);
+        }
+        near = s < 0.5f;
+    }
+    for (;;) {
+        const StepPoint at = step_point<false>(g, s);
+        const bool settled = far_step(far, store, dem, g, at.p, at.minus_inv, s);
+        if (kCount && settled) ++steps, ++visits;
+        if (__any_sync(0xffffffffu, !settled)) {
+            const float s_end = store.get(RayStore::kEnd);
+            if (!settled && s <= s_end)
+                slow_step<kCount, kNearFirst>(far, store, table, dem, g, at, pass_index, s_end, s,
+                                              visits, samples, steps, tracker);
+            if (!__any_sync(0xffffffffu, s <= s_end)) break;
+        }
+    }
+    return store.get(RayStore::kCurrent);
 }
 
 }  // namespace ls200
