@@ -22,7 +22,7 @@
 // a tile on a B200.  Now encode, scan and pack take 41 + 8 + 12 us (the encode
 // kernel 2.3 TB/s of reads, bound by its instructions: 45 groups x ~35 per
 // warp) and decode 99 us.
-#include "internal.cuh"
+#include "staging.cuh"
 
 #include <vector>
 
@@ -246,6 +246,7 @@ static float elevation_scale() { return 50.0f / 32767.0f; }
 
 struct CodecBuffers {
     DeviceBuffer slots, lengths, offsets, total, payload, degrees, error;
+    StagedCopies staged;
 };
 
 static CodecBuffers &codec_buffers(ls200_context *ctx) {
@@ -349,8 +350,7 @@ ls200_status ls200_cbin_decode(ls200_context *ctx, const uint8_t *payload, int64
         b.lengths.reserve(sizeof(int) * kCodecPixels);
         b.degrees.reserve(n);
         b.error.reserve(sizeof(int));
-        LS_CUDA(cudaMemcpyAsync(b.payload.ptr, payload, size_t(size), cudaMemcpyHostToDevice,
-                                ctx->stream));
+        b.staged.to_device(ctx->device, b.payload.ptr, payload, size_t(size), ctx->stream);
         LS_CUDA(cudaMemcpyAsync(b.offsets.ptr, starts.data(), sizeof(long long) * kCodecPixels,
                                 cudaMemcpyHostToDevice, ctx->stream));
         LS_CUDA(cudaMemcpyAsync(b.lengths.ptr, lengths.data(), sizeof(int) * kCodecPixels,
@@ -363,7 +363,7 @@ ls200_status ls200_cbin_decode(ls200_context *ctx, const uint8_t *payload, int64
         int error = 0;
         LS_CUDA(cudaMemcpyAsync(&error, b.error.ptr, sizeof error, cudaMemcpyDeviceToHost,
                                 ctx->stream));
-        LS_CUDA(cudaMemcpyAsync(degrees, b.degrees.ptr, n, cudaMemcpyDeviceToHost, ctx->stream));
+        b.staged.to_host(ctx->device, degrees, b.degrees.ptr, n, ctx->stream);
         LS_CUDA(cudaStreamSynchronize(ctx->stream));
         LS_REQUIRE(error == 0, "compressed horizon block did not decode to 1440 samples");
     });
