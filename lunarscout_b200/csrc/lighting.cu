@@ -465,6 +465,9 @@ static void signal_bits_launch(ls200_context *ctx, LightingBatch B, int tiles,
 // sample's duration through re; the answer per interval is the maximum over
 // runs.  Durations are summed in sample order in FP64 as the reference does
 // (or read from exact prefix sums when every sample duration is an integer).
+// The bits are read a word at a time, eight words in flight, and only run
+// starts and ends are visited (a bit per step: 1981 us for two patches, one
+// year hourly, 12 windows).
 constexpr int kMaxDurationIntervals = 64;
 
 struct DurationParams {
@@ -485,13 +488,21 @@ __device__ __forceinline__ double run_hours(const DurationParams &P, int first, 
     return sum;
 }
 
+// Start windows of one thread: their maxima stay in registers, and a product
+// with more windows has more threads per pixel.
+constexpr int kThreadIntervals = 4;
+
 __global__ void __launch_bounds__(128) duration_kernel(const __grid_constant__ DurationParams P) {
     const int tile = blockIdx.y;
     const int index = blockIdx.x * blockDim.x + threadIdx.x;
     if (index >= kPatch * kPatch) return;
     const size_t plane = static_cast<size_t>(kPatch) * kPatch;
-    double longest[kMaxDurationIntervals];
-    for (int i = 0; i < P.interval_count; ++i) longest[i] = 0.0;
+    const int interval0 = blockIdx.z * kThreadIntervals;
+    double longest[kThreadIntervals] = {};
+    int2 window[kThreadIntervals];
+#pragma unroll
+    for (int i = 0; i < kThreadIntervals; ++i)  // an empty window for none
+        window[i] = interval0 + i < P.interval_count ? P.windows[interval0 + i] : make_int2(0, 0);
     const bool valid =
         index % kPatch < P.valid[tile].x && index / kPatch < P.valid[tile].y;
     if (valid) {
@@ -501,29 +512,48 @@ __global__ void __launch_bounds__(128) duration_kernel(const __grid_constant__ D
         const uint32_t *row = P.bits + offset;
         const uint32_t *earth_row = P.earth_bits ? P.earth_bits + offset : nullptr;
         int run_start = -1;
-        for (int t = 0; t <= P.time_count; ++t) {
-            const size_t word = static_cast<size_t>(t >> 5) * plane;
-            const bool on = t < P.time_count && ((row[word] >> (t & 31)) & 1u) &&
-                            (!earth_row || ((earth_row[word] >> (t & 31)) & 1u));
-            if (on) {
-                if (run_start < 0) run_start = t;
-                continue;
-            }
-            if (run_start < 0) continue;
-            const int run_end = t - 1;
-            for (int i = 0; i < P.interval_count; ++i) {
-                const int2 w = P.windows[i];
-                const int first = max(run_start, w.x);
-                if (first >= w.y || first > run_end) continue;
+        auto end_run = [&](int run_end) {
+#pragma unroll
+            for (int i = 0; i < kThreadIntervals; ++i) {
+                const int first = max(run_start, window[i].x);
+                if (first >= window[i].y || first > run_end) continue;
                 const double d = run_hours(P, first, run_end);
                 if (d > longest[i]) longest[i] = d;
             }
             run_start = -1;
+        };
+        // Whole words: only the bits where a run starts or ends are visited
+        // (bits at and beyond time_count are zero and end the last run).
+        constexpr int kAhead = 8;  // words loaded together
+        for (int w0 = 0; w0 < P.words; w0 += kAhead) {
+            uint32_t words[kAhead];
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) {
+                const size_t at = static_cast<size_t>(w0 + j) * plane;
+                words[j] = w0 + j < P.words ? __ldg(row + at) : 0u;
+                if (earth_row && w0 + j < P.words) words[j] &= __ldg(earth_row + at);
+            }
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) {
+                if (w0 + j >= P.words) break;
+                const int t0 = (w0 + j) * 32;
+                // Bits that differ from the one before them.
+                uint32_t edges = words[j] ^ ((words[j] << 1) | (run_start >= 0 ? 1u : 0u));
+                while (edges) {
+                    const int bit = __ffs(edges) - 1;
+                    edges &= edges - 1;
+                    if (run_start < 0) run_start = t0 + bit;
+                    else end_run(t0 + bit - 1);
+                }
+            }
         }
+        if (run_start >= 0) end_run(P.time_count - 1);
     }
-    for (int i = 0; i < P.interval_count; ++i) {
+#pragma unroll
+    for (int i = 0; i < kThreadIntervals; ++i) {
+        if (interval0 + i >= P.interval_count) break;
         const double v = P.days ? longest[i] / 24.0 : longest[i];
-        P.out[(static_cast<size_t>(tile) * P.interval_count + i) * plane + index] =
+        P.out[(static_cast<size_t>(tile) * P.interval_count + interval0 + i) * plane + index] =
             static_cast<float>(v);
     }
 }
@@ -560,7 +590,8 @@ void mission_duration_launch(ls200_context *ctx, LightingBatch &B, int tiles,
     P.days = days ? 1 : 0;
     for (int t = 0; t < tiles; ++t)
         P.valid[t] = make_int2(B.tiles[t].valid_width, B.tiles[t].valid_height);
-    duration_kernel<<<dim3(kPatch * kPatch / 128, tiles), 128, 0, ctx->stream>>>(P);
+    const int groups = (interval_count + kThreadIntervals - 1) / kThreadIntervals;
+    duration_kernel<<<dim3(kPatch * kPatch / 128, tiles, groups), 128, 0, ctx->stream>>>(P);
     LS_CUDA(cudaGetLastError());
 }
 
