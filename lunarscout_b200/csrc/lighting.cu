@@ -11,8 +11,13 @@
 // into 12 floats per pixel; the time loop is split into chunks so that a
 // tile's 16384 pixels x T times fill all SMs; one thread owns one pixel of
 // one chunk and writes time-major rows [t, 128*128] (coalesced across the
-// warp).  Many tiles may share one launch (blockIdx.z).
+// warp).  Many tiles may share one launch (blockIdx.z).  Long launches settle
+// the clear samples without their exact direction (staged_samples).
 #define LS200_LIGHTING_KERNELS
+#include <cuda_fp16.h>
+
+#include <algorithm>
+
 #include "internal.cuh"
 #include "lighting.cuh"
 
@@ -122,14 +127,12 @@ __device__ __forceinline__ Frame32 load_frame(const float *frames, size_t pixel)
 constexpr int kWindowBins = 32;
 constexpr int kWindowStride = kWindowBins + 1;
 
-// Stage the bins that positions [k0, k1) of the launch's order read (kSpan
-// bins from each step's first bin: 2 for the margin, 5 for the fraction)
-// into `window`; returns the number staged (0: none) and sets `first`, the
-// window's first bin.  In longitude order the body's azimuth moves
-// monotonically across a chunk, so the bins between those of its first and
-// last steps, plus the span and a margin of 2 on each side, cover it; a step
-// outside them reads its row directly.
-template <int kSpan>
+// Stage the bins that the margins at positions [k0, k1) of the launch's order
+// read (two from each step's first bin) into `window`; returns the number
+// staged (0: none) and sets `first`, the window's first bin.  In longitude
+// order the body's azimuth moves monotonically across a chunk, so the bins
+// between those of its first and last steps, plus the span and a margin of 2
+// on each side, cover it; a step outside them reads its row directly.
 __device__ __forceinline__ int stage_window(const LightingBatch &B, const Frame32 &f,
                                             const float *horizon, int k0, int k1, float *window,
                                             int &first) {
@@ -137,19 +140,19 @@ __device__ __forceinline__ int stage_window(const LightingBatch &B, const Frame3
     float azimuth_deg, elevation;
     const float *v = B.vectors + 3 * static_cast<size_t>(__ldg(B.order + k0));
     body_direction(f, __ldg(v), __ldg(v + 1), __ldg(v + 2), azimuth_deg, elevation);
-    const int a = kSpan == 2 ? margin_position(azimuth_deg).left : sun_position(azimuth_deg).left;
+    const int a = margin_position(azimuth_deg).left;
     v = B.vectors + 3 * static_cast<size_t>(__ldg(B.order + k1 - 1));
     body_direction(f, __ldg(v), __ldg(v + 1), __ldg(v + 2), azimuth_deg, elevation);
-    const int b = kSpan == 2 ? margin_position(azimuth_deg).left : sun_position(azimuth_deg).left;
+    const int b = margin_position(azimuth_deg).left;
     int arc = b - a;
     if (arc < 0) arc += kAzimuths;
     int start = arc <= kAzimuths / 2 ? a : b;
     if (arc > kAzimuths / 2) arc = kAzimuths - arc;
     start -= 2;
     if (start < 0) start += kAzimuths;
-    if (arc + kSpan + 4 > kWindowBins) return 0;
+    if (arc + 6 > kWindowBins) return 0;
     first = start;
-    const int width = arc + kSpan + 4;
+    const int width = arc + 6;
     for (int i = 0; i < width; ++i) {
         int bin = first + i;
         if (bin >= kAzimuths) bin -= kAzimuths;
@@ -164,6 +167,374 @@ static int ordered_chunk(int chunk, int time_count) {
     return std::min(chunk, std::max(16, (kWindowBins - 12) * time_count / kAzimuths));
 }
 
+// ---------------------------------------------------------------------------
+// Ordered launches: settled samples.
+//
+// In longitude order a chunk of steps sees the body move through a narrow
+// window of azimuths, and nearly every sample is clear: the whole disk (or the
+// body's centre) stands well above the horizon around it, or well below.  For
+// those the exact direction (two atan2f, a root: some 150 instructions) and the
+// disk's 16 columns are not needed.  Each thread stages, per horizon bin of its
+// pixel's window, the tangents of the elevation above which the signal is
+// certainly high and below which it is certainly low; a step then rotates the
+// vector into the window's own axes (10 multiply-adds), takes the bin from the
+// sine of the angle to the window's middle and the tangent of the elevation
+// from one reciprocal root, and compares: 30 instructions.  Samples in between
+// (about 3 %) are collected per warp and evaluated by the exact functions, 32
+// at a time.
+//
+// Margins: the approximate direction is within 4e-7 rad (2.3e-5 deg) of the
+// exact one in both its own and the reference's rounding, for bodies at least
+// 50 planet radii away (checked per chunk; nearer ones take the exact path).
+// Taking the angle for its sine is 0.11 bin off at the window's end (8 deg).
+// An entry therefore covers one bin more than a sample reads and is chosen half
+// a bin low.  The elevations keep 1.2e-3 deg (kClear), of which the exact
+// fraction needs 1e-3 to round to 0 or 1 and tan_degrees up to 4e-5.
+constexpr int kEntries = 32;        // staged bins per pixel
+constexpr int kEntryStride = kEntries + 1;
+constexpr int kMaxChunk = 256;      // staged vectors per block
+constexpr float kClear = 1.2e-3f;   // deg
+constexpr float kBinsPerRadian = 229.1831180523293f;  // 1440 / 2 pi
+
+// tan of an elevation in degrees from the fast sine and cosine (each within
+// 5e-7): within 4e-5 deg of the angle.  Beyond 85 deg (a bin may hold any
+// value) the tangent of 85, which entry_limits turns into no limit.
+__device__ __forceinline__ float tan_degrees(float degrees) {
+    const float x = fminf(fmaxf(degrees, -85.0f), 85.0f) * 0.017453292519943295f;
+    return __fdividef(__sinf(x), __cosf(x));
+}
+
+// The limits of one entry: the highest tangent raised and the lowest lowered by
+// a small angle, as halves rounded outwards (11 bits: 2^-10 covers them).
+// `margin` is 1.02 times the angle (up to 0.28 deg): tan(x + m) - tan x =
+// tan m (1 + tan^2 x) / (1 - tan x tan m), and up to tan x = 4 the factor is
+// within 2 % of 1.
+__device__ __forceinline__ __half2 entry_limits(float top, float bottom, float margin) {
+    float high = __fmaf_rn(margin, __fmaf_rn(top, top, 1.0f), top);
+    float low = __fmaf_rn(-margin, __fmaf_rn(bottom, bottom, 1.0f), bottom);
+    high = fabsf(top) < 4.0f ? __fmaf_rn(fabsf(high), 0x1p-10f, high) : INFINITY;
+    low = fabsf(bottom) < 4.0f ? __fmaf_rn(fabsf(low), -0x1p-10f, low) : -INFINITY;
+    return __floats2half2_rn(high, low);
+}
+
+__device__ __forceinline__ float4 horizon_quad(const float *horizon, int bin) {
+    if (bin < 0) bin += kAzimuths;
+    else if (bin >= kAzimuths) bin -= kAzimuths;
+    return __ldg(reinterpret_cast<const float4 *>(horizon + bin));
+}
+
+// One pixel's frame turned so that its first axis is across the window's
+// middle azimuth and its second along it.
+struct WindowAxes {
+    float2 x, y, z, t;     // (across, along) per vector component, translation
+    float ux, uy, uz, ut;  // up
+    float position;        // of the middle, in entries
+};
+
+// A step's vector as the packed arithmetic wants it: (x, x, y, y) and
+// (z, z, the operation's two words).
+struct StagedVector {
+    float4 xy, zw;
+    __device__ __forceinline__ uint2 words() const {
+        return make_uint2(__float_as_uint(zw.z), __float_as_uint(zw.w));
+    }
+    __device__ __forceinline__ float3 vector() const { return make_float3(xy.x, xy.z, zw.x); }
+};
+
+// Sine of the angle from the window's middle and tangent of the elevation;
+// returns whether the body is on the middle's side.
+__device__ __forceinline__ bool approximate_direction(const WindowAxes &w, const StagedVector &v,
+                                                      float &sine, float &tangent) {
+    float2 h = __ffma2_rn(make_float2(v.xy.x, v.xy.y), w.x, w.t);
+    h = __ffma2_rn(make_float2(v.xy.z, v.xy.w), w.y, h);
+    h = __ffma2_rn(make_float2(v.zw.x, v.zw.y), w.z, h);
+    const float up = __fmaf_rn(v.zw.x, w.uz,
+                               __fmaf_rn(v.xy.z, w.uy, __fmaf_rn(v.xy.x, w.ux, w.ut)));
+    const float inverse = rsqrtf(__fmaf_rn(h.x, h.x, h.y * h.y));
+    sine = h.x * inverse;
+    tangent = up * inverse;
+    return h.y > 0.0f;
+}
+
+// Shared memory of a staged launch's block.
+struct StagedBlock {
+    __half2 entries[128 * kEntryStride];   // (high above, low below)
+    float4 vectors[2 * kMaxChunk];
+    uint16_t queue[4][64];                 // undecided samples: step << 5 | lane
+    int far;                               // every vector is 50 radii away
+    __device__ __forceinline__ StagedVector vector(int k) const {
+        return StagedVector{vectors[2 * k], vectors[2 * k + 1]};
+    }
+};
+
+// Stage the thread's entries for the block's `steps` vectors; returns their
+// number (0: nothing is settled).  A sample reads kSpan bins from bin
+// azimuth * 4 - kSpan's offset on (5: the disk's columns, 2: the body's centre).
+// The limits lie `clearance` (deg, small: see entry_limits) above the highest
+// and below the lowest of them, all raised by `shift` (deg, any).
+template <int kSpan>
+__device__ __forceinline__ int stage_entries(StagedBlock &S, const Frame32 &f,
+                                             const float *horizon, int steps, float shift,
+                                             float clearance, WindowAxes &w) {
+    const float3 middle = S.vector(steps >> 1).vector();
+    float azimuth_deg, elevation;
+    body_direction(f, middle.x, middle.y, middle.z, azimuth_deg, elevation);
+    float sin_a = __fmaf_rn(middle.z, f.v[6], __fmaf_rn(middle.y, f.v[3],
+                                                        __fmaf_rn(middle.x, f.v[0], f.v[9])));
+    float cos_a = __fmaf_rn(middle.z, f.v[7], __fmaf_rn(middle.y, f.v[4],
+                                                        __fmaf_rn(middle.x, f.v[1], f.v[10])));
+    const float inverse = rsqrtf(__fmaf_rn(sin_a, sin_a, cos_a * cos_a));
+    sin_a *= inverse;
+    cos_a *= inverse;
+    w.x = make_float2(f.v[0] * cos_a - f.v[1] * sin_a, f.v[0] * sin_a + f.v[1] * cos_a);
+    w.y = make_float2(f.v[3] * cos_a - f.v[4] * sin_a, f.v[3] * sin_a + f.v[4] * cos_a);
+    w.z = make_float2(f.v[6] * cos_a - f.v[7] * sin_a, f.v[6] * sin_a + f.v[7] * cos_a);
+    w.t = make_float2(f.v[9] * cos_a - f.v[10] * sin_a, f.v[9] * sin_a + f.v[10] * cos_a);
+    w.ux = f.v[2], w.uy = f.v[5], w.uz = f.v[8], w.ut = f.v[11];
+    w.position = azimuth_deg * 4.0f - (kSpan == 5 ? 1.58f : 0.0f);
+    float low = w.position, high = w.position;
+#pragma unroll
+    for (int end = 0; end < 2; ++end) {
+        float sine, tangent;
+        if (approximate_direction(w, S.vector(end ? steps - 1 : 0), sine, tangent) &&
+            fabsf(sine) < 0.14f) {
+            low = fminf(low, __fmaf_rn(sine, kBinsPerRadian, w.position));
+            high = fmaxf(high, __fmaf_rn(sine, kBinsPerRadian, w.position));
+        }
+    }
+    // Whole quads of bins from two below the lowest position; steps that fall
+    // outside the entries are evaluated exactly.
+    const int first = (static_cast<int>(floorf(low)) - 2) & ~3;
+    const int count = min(kEntries, static_cast<int>(floorf(high)) + 3 - first);
+    w.position -= static_cast<float>(first) + 0.5f;
+    const float margin = 1.02f * 0.017453292519943295f * clearance;
+    __half2 *entries = S.entries + threadIdx.x * kEntryStride;
+    float bins[9];  // tangents of the horizon from entry e's bin on
+    float sum = 0.0f;
+    auto take = [&](int at, float4 h) {
+        sum = (h.x + h.y) + (h.z + h.w);
+        bins[at] = tan_degrees(h.x + shift);
+        bins[at + 1] = tan_degrees(h.y + shift);
+        bins[at + 2] = tan_degrees(h.z + shift);
+        bins[at + 3] = tan_degrees(h.w + shift);
+    };
+    take(0, horizon_quad(horizon, first));
+    float sum0 = sum;
+    take(4, horizon_quad(horizon, first + 4));
+    float sum1 = sum;
+    float4 next = horizon_quad(horizon, first + 8);
+    int bin0 = first < 0 ? first + kAzimuths : first;
+    for (int e = 0; e < count; e += 4) {
+        const float4 c = next;
+        next = horizon_quad(horizon, first + e + 12);
+        bins[8] = tan_degrees(c.x + shift);
+        const float sum2 = (c.x + c.y) + (c.z + c.w);
+        const bool finite = fabsf(sum0 + sum1 + sum2) < 1e6f;
+        // The disk's first bin below azimuth 0.395 deg is special (its columns
+        // extrapolate): bins 1437 to 1439 settle nothing.
+        const bool seam = kSpan == 5 && bin0 == kAzimuths - 4;
+        float most[8], least[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            most[k] = fmaxf(bins[k], bins[k + 1]);
+            least[k] = fminf(bins[k], bins[k + 1]);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            float top, bottom;
+            if (kSpan == 5) {  // bins k .. k + 5
+                top = fmaxf(fmaxf(most[k], most[k + 2]), most[k + 4]);
+                bottom = fminf(fminf(least[k], least[k + 2]), least[k + 4]);
+            } else {           // bins k .. k + 2
+                top = fmaxf(most[k], most[k + 1]);
+                bottom = fminf(least[k], least[k + 1]);
+            }
+            __half2 limits = entry_limits(top, bottom, margin);
+            if (!finite || (seam && k > 0)) limits = __floats2half2_rn(INFINITY, -INFINITY);
+            entries[e + k] = limits;
+        }
+        sum0 = sum1;
+        sum1 = sum2;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) bins[k] = bins[k + 4];
+        bins[4] = bins[8];
+        bins[5] = tan_degrees(c.y + shift);
+        bins[6] = tan_degrees(c.z + shift);
+        bins[7] = tan_degrees(c.w + shift);
+        bin0 = bin0 + 4 >= kAzimuths ? bin0 + 4 - kAzimuths : bin0 + 4;
+    }
+    return S.far ? count : 0;
+}
+
+// The block's vectors for positions [k0, k0 + steps) of the launch's order,
+// with the operation's words for each time index.
+template <class Op>
+__device__ __forceinline__ void stage_vectors(StagedBlock &S, const LightingBatch &B, int k0,
+                                              int steps, const Op &op) {
+    if (threadIdx.x == 0) S.far = 1;
+    __syncthreads();
+    const float scale = 1.0f / (50.0f * fabsf(static_cast<float>(B.tiles[blockIdx.z].proj[0])) +
+                                1.0f);
+    for (int k = threadIdx.x; k < steps; k += blockDim.x) {
+        const int t = __ldg(B.order + k0 + k);
+        const float *v = B.vectors + 3 * static_cast<size_t>(t);
+        const float x = __ldg(v), y = __ldg(v + 1), z = __ldg(v + 2);
+        const uint2 words = op.words(t);
+        S.vectors[2 * k] = make_float4(x, x, y, y);
+        S.vectors[2 * k + 1] =
+            make_float4(z, z, __uint_as_float(words.x), __uint_as_float(words.y));
+        const float sx = x * scale, sy = y * scale, sz = z * scale;
+        if (!(sx * sx + sy * sy + sz * sz >= 1.0f)) S.far = 0;
+    }
+    __syncthreads();
+}
+
+// Visits every sample of the block: op.settled(words, high) where the entries
+// decide the thread's own pixel, op.outside(words) where that lies outside the
+// valid rectangle (!valid), and op.exact(pixel offset, frame, horizon, vector,
+// words) otherwise, for a pixel of the thread's warp.
+template <int kSpan, class Op>
+__device__ __forceinline__ void staged_samples(StagedBlock &S, const LightingBatch &B, bool valid,
+                                               float shift, float clearance, Op &op) {
+    const int lane = threadIdx.x & 31;
+    const size_t pixel = static_cast<size_t>(blockIdx.z) * kPatch * kPatch +
+                         blockIdx.x * 128 + threadIdx.x;
+    uint16_t *queue = S.queue[threadIdx.x >> 5];
+    const int k0 = blockIdx.y * B.chunk;
+    const int steps = min(B.chunk, B.time_count - k0);
+    stage_vectors(S, B, k0, steps, op);
+    WindowAxes w{};
+    int count = 0;
+    if (valid)
+        count = stage_entries<kSpan>(S, load_frame(B.frames, pixel),
+                                     B.horizons + pixel * kAzimuths, steps, shift, clearance, w);
+    const __half2 *entries = S.entries + threadIdx.x * kEntryStride;
+    int pending = 0;  // queued samples of the warp
+    for (int first = 0; first < steps; first += 32) {
+        const int group = min(32, steps - first);
+        uint32_t undecided = 0;  // of the group's steps
+        if (valid) {
+#pragma unroll 4
+            for (int j = 0; j < group; ++j) {
+                const StagedVector v = S.vector(first + j);
+                float sine, tangent;
+                const bool ahead = approximate_direction(w, v, sine, tangent);
+                const int e = __float2int_rd(__fmaf_rn(sine, kBinsPerRadian, w.position));
+                const bool staged =
+                    static_cast<unsigned>(e) < static_cast<unsigned>(count) && ahead;
+                float2 limits = make_float2(0.0f, 0.0f);
+                if (staged) limits = __half22float2(entries[e]);
+                const bool high = staged && tangent > limits.x;
+                const bool low = staged && tangent < limits.y;
+                if (high || low) op.settled(v.words(), high);
+                else undecided |= 1u << j;
+            }
+        } else {
+            for (int j = 0; j < group; ++j) op.outside(S.vector(first + j).words());
+        }
+        // Queue the undecided, one of each lane a round, and evaluate them
+        // whenever a warp's worth (or, at the end, the rest) is there.
+        const bool last = first + 32 >= steps;
+        for (;;) {
+            const unsigned from = __ballot_sync(0xffffffffu, undecided != 0);
+            if (undecided) {
+                const int j = __ffs(undecided) - 1;
+                undecided &= undecided - 1;
+                queue[pending + __popc(from & ((1u << lane) - 1u))] =
+                    static_cast<uint16_t>((first + j) << 5 | lane);
+            }
+            pending += __popc(from);
+            if (pending < 32 && (from || !last || !pending)) {
+                if (!from) break;
+                continue;
+            }
+            const int n = min(pending, 32);
+            __syncwarp();
+            if (lane < n) {
+                const int entry = queue[lane];
+                const int offset = (entry & 31) - lane;
+                const StagedVector v = S.vector(entry >> 5);
+                op.exact(offset, load_frame(B.frames, pixel + offset),
+                         B.horizons + (pixel + offset) * kAzimuths, v.vector(), v.words());
+            }
+            __syncwarp();
+            if (lane + n < pending) queue[lane] = queue[lane + n];
+            pending -= n;
+            __syncwarp();
+        }
+    }
+}
+
+// Longest chunk of a staged launch: about 20 bins of azimuth, so that its
+// entries fit.  Launches below kStagedSteps steps spend more on staging than
+// they save: one patch takes 212 us against 342 at 720 steps, 236 either way
+// at 360.
+static int staged_chunk(int time_count) {
+    return std::max(4, std::min(kMaxChunk, static_cast<int>(20ll * time_count / kAzimuths)));
+}
+constexpr int kStagedSteps = 720;
+// (Rows are staged in 16-byte quads, and a word plane's 32-bit offset bounds
+// the bits' time axis to 2^22 steps.)
+static bool staged_launch(const LightingBatch &B) {
+    return B.order && B.time_count >= kStagedSteps && B.time_count < (1 << 22) &&
+           (reinterpret_cast<uintptr_t>(B.horizons) & 15) == 0;
+}
+
+// Fractions (float32 or bytes) into the launch's time-major output; the words
+// of a step are its plane's 64-bit offset.
+template <class T>
+struct StoreSample {
+    T *out;  // the thread's pixel in the first plane
+    int time_start;
+    __device__ __forceinline__ uint2 words(int t) const {
+        const unsigned long long offset =
+            static_cast<unsigned long long>(t - time_start) * (kPatch * kPatch);
+        return make_uint2(static_cast<unsigned>(offset), static_cast<unsigned>(offset >> 32));
+    }
+    __device__ __forceinline__ T *place(uint2 w) const {
+        return out + (static_cast<unsigned long long>(w.y) << 32 | w.x);
+    }
+    static __device__ __forceinline__ T value(float visible) {
+        return sizeof(T) == 1 ? static_cast<T>(static_cast<int>(__fmul_rn(255.0f, visible)))
+                              : static_cast<T>(visible);
+    }
+    __device__ __forceinline__ void settled(uint2 w, bool high) const {
+        *place(w) = high ? static_cast<T>(sizeof(T) == 1 ? 255 : 1) : static_cast<T>(0);
+    }
+    __device__ __forceinline__ void outside(uint2 w) const { *place(w) = static_cast<T>(0); }
+    __device__ __forceinline__ void exact(int offset, const Frame32 &f, const float *horizon,
+                                          float3 v, uint2 w) const {
+        float azimuth_deg, elevation;
+        body_direction(f, v.x, v.y, v.z, azimuth_deg, elevation);
+        place(w)[offset] = value(sun_fraction(horizon, azimuth_deg, elevation));
+    }
+};
+
+// Blocks per SM of the staged kernels: 7 (72 registers) took 2.08 ms for four
+// patches of a year's hourly bytes, 8 (64, a few spills) 2.13.
+constexpr int kStagedBlocks = 7;
+
+// Sun fractions of an ordered launch.  Four patches, 8761 steps, bytes (B200,
+// whole call): 5.66 ms with the exact functions for every sample, 2.08 ms.  A
+// warp's step takes 48 instructions with its share of exact samples (about 14),
+// a chunk's staging 2300; 78 % of the issue slots are busy.
+template <class T>
+__global__ void __launch_bounds__(128, kStagedBlocks)
+    staged_fraction_kernel(const __grid_constant__ LightingBatch B) {
+    __shared__ StagedBlock S;
+    const TileGeo &g = B.tiles[blockIdx.z];
+    const int index = blockIdx.x * 128 + threadIdx.x;
+    const bool valid = index % kPatch < g.valid_width && index / kPatch < g.valid_height;
+    StoreSample<T> op{static_cast<T *>(B.out) +
+                          static_cast<size_t>(blockIdx.z) * B.time_count * (kPatch * kPatch) +
+                          index,
+                      B.time_start};
+    staged_samples<5>(S, B, valid, 0.0f, c_half_circle[7] + kClear, op);
+}
+
+// Margins, and fractions of launches that are not staged.  Margins stage each
+// chunk's bins (stage_window); a short or unordered launch of fractions reads
+// its rows directly.
 template <int kSignal>
 __global__ void __launch_bounds__(128) lighting_kernel(const __grid_constant__ LightingBatch B) {
     const int tile = blockIdx.z;
@@ -185,35 +556,30 @@ __global__ void __launch_bounds__(128) lighting_kernel(const __grid_constant__ L
         }
         return;
     }
-    Frame32 f;
-    const float *src = B.frames + (static_cast<size_t>(tile) * plane + index) * 12;
-#pragma unroll
-    for (int k = 0; k < 12; ++k) f.v[k] = src[k];
-    const float *horizon = B.horizons + (static_cast<size_t>(tile) * plane + index) * kAzimuths;
-    __shared__ float windows[128 * kWindowStride];
-    float *window = windows + threadIdx.x * kWindowStride;
-    constexpr int kSpan = kSignal == kSignalMargin ? 2 : 5;
+    const size_t pixel = static_cast<size_t>(tile) * plane + index;
+    const Frame32 f = load_frame(B.frames, pixel);
+    const float *horizon = B.horizons + pixel * kAzimuths;
+    constexpr bool kMargin = kSignal == kSignalMargin;
+    __shared__ float windows[kMargin ? 128 * kWindowStride : 1];
+    float *window = windows + (kMargin ? threadIdx.x * kWindowStride : 0);
     int first = 0;
-    const int width = stage_window<kSpan>(B, f, horizon, k0, k1, window, first);
+    const int width = kMargin ? stage_window(B, f, horizon, k0, k1, window, first) : 0;
     for (int k = k0; k < k1; ++k) {
         const int t = B.order ? __ldg(B.order + k) : B.time_start + k;
         const float *v = B.vectors + 3 * static_cast<size_t>(t);
         float azimuth_deg, elevation;
         body_direction(f, __ldg(v), __ldg(v + 1), __ldg(v + 2), azimuth_deg, elevation);
         const size_t o = tile_out + static_cast<size_t>(t - B.time_start) * plane + index;
-        const BinPosition p = kSignal == kSignalMargin ? margin_position(azimuth_deg)
-                                                       : sun_position(azimuth_deg);
-        int offset = p.left - first;
-        if (offset < 0) offset += kAzimuths;
-        const bool staged = offset + kSpan <= width;
-        if (kSignal == kSignalMargin) {
+        if (kMargin) {
+            const BinPosition p = margin_position(azimuth_deg);
+            int offset = p.left - first;
+            if (offset < 0) offset += kAzimuths;
             static_cast<float *>(B.out)[o] =
-                staged ? horizon_margin_bins(SharedBins{window, offset}, p.fraction, elevation)
-                       : horizon_margin_bins(GlobalBins{horizon, p.left}, p.fraction, elevation);
+                offset + 2 <= width
+                    ? horizon_margin_bins(SharedBins{window, offset}, p.fraction, elevation)
+                    : horizon_margin_bins(GlobalBins{horizon, p.left}, p.fraction, elevation);
         } else {
-            const float visible =
-                staged ? sun_fraction_bins(SharedBins{window, offset}, p.fraction, elevation)
-                       : sun_fraction_bins(GlobalBins{horizon, p.left}, p.fraction, elevation);
+            const float visible = sun_fraction(horizon, azimuth_deg, elevation);
             if (kSignal == kSignalBytes)
                 static_cast<uint8_t *>(B.out)[o] =
                     static_cast<uint8_t>(static_cast<int>(__fmul_rn(255.0f, visible)));
@@ -284,11 +650,13 @@ __global__ void sun_fraction_kernel(const float *horizons, const float *azimuth_
 
 int lighting_chunk(ls200_context *ctx, int tiles, int time_count) {
     // Enough (pixel-block x chunk x tile) blocks for ~8 waves of 128-thread
-    // blocks on every SM, chunks of at least 16 time steps.
+    // blocks on every SM, chunks of at least 4 time steps (a short table's
+    // launch is bound by the latency of its row reads: 125 steps of one patch
+    // took 56 us in chunks of 16, 47 in chunks of 5: 32-byte sectors of 2 M rows).
     const int blocks_per_chunk = (kPatch * kPatch / 128) * tiles;
     const int want = ctx->props.multiProcessorCount * 16 * 8;
     int chunks = std::max(1, want / std::max(1, blocks_per_chunk));
-    chunks = std::min(chunks, std::max(1, time_count / 16));
+    chunks = std::min(chunks, std::max(1, time_count / 4));
     return (time_count + chunks - 1) / chunks;
 }
 
@@ -344,6 +712,13 @@ void lighting_launch(ls200_context *ctx, LightingBatch &B, int tiles, int signal
     if (signal == kSignalPsr) {
         dim3 grid(kPatch * kPatch / kPsrWarps, 1, tiles);
         psr_kernel<<<grid, kPsrWarps * 32, 0, ctx->stream>>>(B);
+    } else if (staged_launch(B) && signal != kSignalMargin) {
+        B.chunk = staged_chunk(B.time_count);
+        dim3 grid(kPatch * kPatch / 128, (B.time_count + B.chunk - 1) / B.chunk, tiles);
+        if (signal == kSignalBytes)
+            staged_fraction_kernel<uint8_t><<<grid, 128, 0, ctx->stream>>>(B);
+        else
+            staged_fraction_kernel<float><<<grid, 128, 0, ctx->stream>>>(B);
     } else {
         B.chunk = lighting_chunk(ctx, tiles, B.time_count);
         if (B.order) B.chunk = ordered_chunk(B.chunk, B.time_count);
@@ -395,71 +770,86 @@ void directions_launch(ls200_context *ctx, LightingBatch &B, int tiles, float2 *
     LS_CUDA(cudaGetLastError());
 }
 
-// Sun fraction at (azimuth, elevation) from a thread's staged window when it
-// holds the five bins, else from the pixel's row.
-__device__ __forceinline__ float staged_sun_fraction(const float *window, int first, int width,
-                                                     const float *horizon, float azimuth_deg,
-                                                     float elevation) {
-    const BinPosition p = sun_position(azimuth_deg);
-    int offset = p.left - first;
-    if (offset < 0) offset += kAzimuths;
-    return offset + 5 <= width
-               ? sun_fraction_bins(SharedBins{window, offset}, p.fraction, elevation)
-               : sun_fraction_bins(GlobalBins{horizon, p.left}, p.fraction, elevation);
-}
-
-// The same for the margin (two bins).
-__device__ __forceinline__ float staged_margin(const float *window, int first, int width,
-                                               const float *horizon, float azimuth_deg,
-                                               float elevation) {
-    const BinPosition p = margin_position(azimuth_deg);
-    int offset = p.left - first;
-    if (offset < 0) offset += kAzimuths;
-    return offset + 2 <= width
-               ? horizon_margin_bins(SharedBins{window, offset}, p.fraction, elevation)
-               : horizon_margin_bins(GlobalBins{horizon, p.left}, p.fraction, elevation);
-}
-
 // Threshold bits of one signal of one body, word-major [tiles, words, 16384]
 // (zeroed before the launch): bit t is set where signal >= threshold
 // (kAtLeast) or signal < threshold.  kSpan 5 is the sun fraction, 2 the
 // margin.  Each thread visits a chunk of the body's table in its longitude
-// order with the chunk's bins staged, and sets the bits of its steps with
-// atomicOr (other chunks own the word's other steps).  Each signal runs in
-// its own body's order, so the Earth's reads are staged as well as the Sun's.
+// order and sets the bits of its steps with atomicOr (other chunks own the
+// word's other steps).  Each signal runs in its own body's order.
+template <int kSpan>
+__device__ __forceinline__ float signal_value(const float *horizon, float azimuth_deg,
+                                              float elevation) {
+    return kSpan == 5 ? sun_fraction(horizon, azimuth_deg, elevation)
+                      : horizon_margin(horizon, azimuth_deg, elevation);
+}
+
+template <bool kAtLeast>
+__device__ __forceinline__ bool passes(float value, float threshold) {
+    return kAtLeast ? value >= threshold : value < threshold;
+}
+
+// The words of a step: the offset of its word's plane, and its bit.
+template <int kSpan, bool kAtLeast>
+struct SetBit {
+    uint32_t *bits;  // the thread's pixel in the first word plane
+    float threshold;
+    bool high, low;  // the bit of a settled high or low signal
+    __device__ __forceinline__ uint2 words(int t) const {
+        return make_uint2(static_cast<unsigned>(t >> 5) * (kPatch * kPatch), 1u << (t & 31));
+    }
+    __device__ __forceinline__ void settled(uint2 w, bool is_high) const {
+        if (is_high ? high : low) atomicOr(bits + w.x, w.y);
+    }
+    __device__ __forceinline__ void outside(uint2) const {}
+    __device__ __forceinline__ void exact(int offset, const Frame32 &f, const float *horizon,
+                                          float3 v, uint2 w) const {
+        float azimuth_deg, elevation;
+        body_direction(f, v.x, v.y, v.z, azimuth_deg, elevation);
+        if (passes<kAtLeast>(signal_value<kSpan>(horizon, azimuth_deg, elevation), threshold))
+            atomicOr(bits + offset + w.x, w.y);
+    }
+};
+
+template <int kSpan, bool kAtLeast>
+__global__ void __launch_bounds__(128, kStagedBlocks)
+    staged_bits_kernel(const __grid_constant__ LightingBatch B, float threshold, int words,
+                       uint32_t *__restrict__ bits) {
+    __shared__ StagedBlock S;
+    const TileGeo &g = B.tiles[blockIdx.z];
+    const int index = blockIdx.x * 128 + threadIdx.x;
+    const bool valid = index % kPatch < g.valid_width && index / kPatch < g.valid_height;
+    // A settled margin is above or below the threshold itself.
+    SetBit<kSpan, kAtLeast> op{
+        bits + static_cast<size_t>(blockIdx.z) * words * (kPatch * kPatch) + index, threshold,
+        kSpan == 5 ? passes<kAtLeast>(1.0f, threshold) : kAtLeast,
+        kSpan == 5 ? passes<kAtLeast>(0.0f, threshold) : !kAtLeast};
+    staged_samples<kSpan>(S, B, valid, kSpan == 5 ? 0.0f : threshold,
+                          kSpan == 5 ? c_half_circle[7] + kClear : kClear, op);
+}
+
+// The same without an order, or for a short table: every sample exactly.
 template <int kSpan, bool kAtLeast>
 __global__ void __launch_bounds__(128) signal_bits_kernel(const __grid_constant__ LightingBatch B,
                                                           float threshold, int words,
                                                           uint32_t *__restrict__ bits) {
     const int tile = blockIdx.z;
     const int index = blockIdx.x * blockDim.x + threadIdx.x;
-    if (index >= kPatch * kPatch) return;
     const TileGeo &g = B.tiles[tile];
-    const int sample = index % kPatch, line = index / kPatch;
-    if (sample >= g.valid_width || line >= g.valid_height) return;
+    if (index % kPatch >= g.valid_width || index / kPatch >= g.valid_height) return;
     const size_t plane = static_cast<size_t>(kPatch) * kPatch;
     uint32_t *tile_bits = bits + static_cast<size_t>(tile) * words * plane + index;
     const int k0 = blockIdx.y * B.chunk;
     const int k1 = min(k0 + B.chunk, B.time_count);
-    Frame32 f;
-    const float *src = B.frames + (static_cast<size_t>(tile) * plane + index) * 12;
-#pragma unroll
-    for (int k = 0; k < 12; ++k) f.v[k] = src[k];
-    const float *horizon = B.horizons + (static_cast<size_t>(tile) * plane + index) * kAzimuths;
-    __shared__ float windows[128 * kWindowStride];
-    float *window = windows + threadIdx.x * kWindowStride;
-    int first = 0;
-    const int width = stage_window<kSpan>(B, f, horizon, k0, k1, window, first);
+    const size_t pixel = static_cast<size_t>(tile) * plane + index;
+    const Frame32 f = load_frame(B.frames, pixel);
+    const float *horizon = B.horizons + pixel * kAzimuths;
     for (int k = k0; k < k1; ++k) {
         const int t = B.order ? __ldg(B.order + k) : k;
         const float *v = B.vectors + 3 * static_cast<size_t>(t);
         float azimuth_deg, elevation;
         body_direction(f, __ldg(v), __ldg(v + 1), __ldg(v + 2), azimuth_deg, elevation);
-        const float value =
-            kSpan == 5 ? staged_sun_fraction(window, first, width, horizon, azimuth_deg, elevation)
-                       : staged_margin(window, first, width, horizon, azimuth_deg, elevation);
-        const bool on = kAtLeast ? value >= threshold : value < threshold;
-        if (on) atomicOr(tile_bits + static_cast<size_t>(t >> 5) * plane, 1u << (t & 31));
+        if (passes<kAtLeast>(signal_value<kSpan>(horizon, azimuth_deg, elevation), threshold))
+            atomicOr(tile_bits + static_cast<size_t>(t >> 5) * plane, 1u << (t & 31));
     }
 }
 
@@ -475,10 +865,15 @@ static void signal_bits_launch(ls200_context *ctx, LightingBatch B, int tiles,
                             ctx->stream));
     B.vectors = vectors;
     B.order = order;
-    B.chunk = lighting_chunk(ctx, tiles, B.time_count);
-    if (B.order) B.chunk = ordered_chunk(B.chunk, B.time_count);
+    const bool staged = staged_launch(B);
+    B.chunk = staged ? staged_chunk(B.time_count) : lighting_chunk(ctx, tiles, B.time_count);
     dim3 grid(kPatch * kPatch / 128, (B.time_count + B.chunk - 1) / B.chunk, tiles);
-    signal_bits_kernel<kSpan, kAtLeast><<<grid, 128, 0, ctx->stream>>>(B, threshold, words, bits);
+    if (staged)
+        staged_bits_kernel<kSpan, kAtLeast>
+            <<<grid, 128, 0, ctx->stream>>>(B, threshold, words, bits);
+    else
+        signal_bits_kernel<kSpan, kAtLeast>
+            <<<grid, 128, 0, ctx->stream>>>(B, threshold, words, bits);
     LS_CUDA(cudaGetLastError());
 }
 
@@ -759,44 +1154,57 @@ void safe_haven_launch(ls200_context *ctx, LightingBatch &B, int tiles, const fl
 // threshold.  Each thread counts its pixel over one time chunk and adds the
 // count to the pixel's counter; visibility_finalize divides by T (FP64, then
 // rounded to float32).
+struct CountVisible {
+    unsigned *counts;  // the thread's pixel
+    float threshold;
+    unsigned count;
+    __device__ __forceinline__ uint2 words(int) const { return make_uint2(0u, 0u); }
+    __device__ __forceinline__ void settled(uint2, bool high) { count += high ? 1u : 0u; }
+    __device__ __forceinline__ void outside(uint2) const {}
+    __device__ __forceinline__ void exact(int offset, const Frame32 &f, const float *horizon,
+                                          float3 v, uint2) const {
+        float azimuth_deg, elevation;
+        body_direction(f, v.x, v.y, v.z, azimuth_deg, elevation);
+        if (horizon_margin(horizon, azimuth_deg, elevation) >= threshold)
+            atomicAdd(counts + offset, 1u);
+    }
+};
+
+__global__ void __launch_bounds__(128, kStagedBlocks)
+    staged_visibility_kernel(const __grid_constant__ LightingBatch B, float threshold,
+                             unsigned *__restrict__ counts) {
+    __shared__ StagedBlock S;
+    const TileGeo &g = B.tiles[blockIdx.z];
+    const int index = blockIdx.x * 128 + threadIdx.x;
+    const bool valid = index % kPatch < g.valid_width && index / kPatch < g.valid_height;
+    CountVisible op{counts + static_cast<size_t>(blockIdx.z) * (kPatch * kPatch) + index,
+                    threshold, 0u};
+    staged_samples<2>(S, B, valid, threshold, kClear, op);
+    if (op.count) atomicAdd(op.counts, op.count);
+}
+
+// The same without an order, or for a short table: every sample exactly.
 __global__ void __launch_bounds__(128) visibility_kernel(const __grid_constant__ LightingBatch B,
                                                          float threshold,
                                                          unsigned *__restrict__ counts) {
     const int tile = blockIdx.z;
     const int index = blockIdx.x * blockDim.x + threadIdx.x;
-    if (index >= kPatch * kPatch) return;
     const TileGeo &g = B.tiles[tile];
     if (index % kPatch >= g.valid_width || index / kPatch >= g.valid_height) return;
-    const size_t plane = static_cast<size_t>(kPatch) * kPatch;
     const int k0 = blockIdx.y * B.chunk;
     const int k1 = min(k0 + B.chunk, B.time_count);
-    Frame32 f;
-    const float *src = B.frames + (static_cast<size_t>(tile) * plane + index) * 12;
-#pragma unroll
-    for (int k = 0; k < 12; ++k) f.v[k] = src[k];
-    const float *horizon = B.horizons + (static_cast<size_t>(tile) * plane + index) * kAzimuths;
-    // A count does not depend on the order of its steps: visit them in the
-    // table's longitude order with the chunk's bins staged (as lighting_kernel).
-    __shared__ float windows[128 * kWindowStride];
-    float *window = windows + threadIdx.x * kWindowStride;
-    int first = 0;
-    const int width = stage_window<2>(B, f, horizon, k0, k1, window, first);
+    const size_t pixel = static_cast<size_t>(tile) * kPatch * kPatch + index;
+    const Frame32 f = load_frame(B.frames, pixel);
+    const float *horizon = B.horizons + pixel * kAzimuths;
     unsigned count = 0;
     for (int k = k0; k < k1; ++k) {
         const int t = B.order ? __ldg(B.order + k) : k;
         const float *v = B.vectors + 3 * static_cast<size_t>(t);
         float azimuth_deg, elevation;
         body_direction(f, __ldg(v), __ldg(v + 1), __ldg(v + 2), azimuth_deg, elevation);
-        const BinPosition p = margin_position(azimuth_deg);
-        int offset = p.left - first;
-        if (offset < 0) offset += kAzimuths;
-        const float margin =
-            offset + 2 <= width
-                ? horizon_margin_bins(SharedBins{window, offset}, p.fraction, elevation)
-                : horizon_margin_bins(GlobalBins{horizon, p.left}, p.fraction, elevation);
-        count += margin >= threshold ? 1u : 0u;
+        count += horizon_margin(horizon, azimuth_deg, elevation) >= threshold ? 1u : 0u;
     }
-    if (count) atomicAdd(counts + static_cast<size_t>(tile) * plane + index, count);
+    if (count) atomicAdd(counts + pixel, count);
 }
 
 __global__ void visibility_finalize(const unsigned *__restrict__ counts, int n, int time_count,
@@ -819,10 +1227,13 @@ void visibility_launch(ls200_context *ctx, LightingBatch &B, int tiles, float th
     dim3 grid_frames(kPatch * kPatch / 128, tiles);
     frames_kernel<<<grid_frames, 128, 0, ctx->stream>>>(B);
     LS_CUDA(cudaGetLastError());
-    B.chunk = lighting_chunk(ctx, tiles, B.time_count);
-    if (B.order) B.chunk = ordered_chunk(B.chunk, B.time_count);
+    const bool staged = staged_launch(B);
+    B.chunk = staged ? staged_chunk(B.time_count) : lighting_chunk(ctx, tiles, B.time_count);
     dim3 grid(kPatch * kPatch / 128, (B.time_count + B.chunk - 1) / B.chunk, tiles);
-    visibility_kernel<<<grid, 128, 0, ctx->stream>>>(B, threshold, counts);
+    if (staged)
+        staged_visibility_kernel<<<grid, 128, 0, ctx->stream>>>(B, threshold, counts);
+    else
+        visibility_kernel<<<grid, 128, 0, ctx->stream>>>(B, threshold, counts);
     LS_CUDA(cudaGetLastError());
     visibility_finalize<<<(n + 255) / 256, 256, 0, ctx->stream>>>(counts, n, B.time_count, valid,
                                                                   out);

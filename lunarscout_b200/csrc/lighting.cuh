@@ -127,8 +127,8 @@ __device__ __forceinline__ void body_direction(const Frame32 &f, float vx, float
 }
 
 // The signals read the horizon bins left, left+1, ... (wrapped at 1440)
-// through a bin accessor: GlobalBins reads the pixel's row, SharedBins a
-// window of it staged in shared memory.  Both return the same values.
+// through a bin accessor: GlobalBins reads the pixel's row, SharedBins (the
+// margins) a window of it staged in shared memory.  Both return the same values.
 struct GlobalBins {
     const float *horizon;
     int left;
