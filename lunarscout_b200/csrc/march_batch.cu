@@ -9,7 +9,9 @@
 // transpose.
 //
 // Traversal 0 is the reference traversal (march_core.cuh), bit-identical to
-// the per-tile kernel.  Traversal 1 adds the skip ladder (ladder_advance):
+// the per-tile kernel and, as there, with most steps settled without the full
+// arithmetic (march_near, march_dem_far: two sites of 2048^2 pixels over
+// 3072^2, 318 -> 208 ms).  Traversal 1 adds the skip ladder (ladder_advance):
 // a cull climbs to the largest culled ancestor cell, which removes most of
 // the footprint-limited steps of long rays; its results are checked against
 // its own CPU restatement (oracle flag OPT_LADDER) and their distance from
@@ -18,7 +20,7 @@
 // Launch configuration (autotuned, never changing results): how the 32 lanes
 // of a job map onto rays (L adjacent pixels x 32/L adjacent azimuths, L a
 // power of two up to 32), and the resident blocks per SM (8 at 64 registers,
-// 6 at 80).
+// 6 at 80; the relative march takes 7 for 8).
 #include "march_core.cuh"
 
 #include <map>
@@ -80,6 +82,27 @@ struct GlobalLevels {
     __device__ __forceinline__ int4 cells(int l) const { return __ldg(&t->cells[l]); }
 };
 
+// A warp's copy of its DEM's level table in shared memory (each warp may be on
+// a different DEM).
+struct WarpDem {
+    LevelTable table;
+    float2 last;  // width - 1, height - 1
+};
+struct WarpLevels {
+    const LevelTable &t;
+    const float2 &last_cell;
+    __device__ __forceinline__ float2 last() const { return last_cell; }
+    __device__ __forceinline__ float side(int l) const { return t.side[l]; }
+    __device__ __forceinline__ float fallback(int l) const { return t.fallback[l]; }
+    __device__ __forceinline__ float out_step(int l) const { return t.out_step[l]; }
+    __device__ __forceinline__ int4 cells(int l) const { return t.cells[l]; }
+};
+
+struct SitesBlock {
+    RayStore::Block rays;
+    WarpDem dems[4];
+};
+
 __global__ void batch_dem_kernel(const BatchDemSource *__restrict__ sources,
                                  BatchDem *__restrict__ dems) {
     const BatchDemSource &s = sources[blockIdx.x];
@@ -108,7 +131,8 @@ __global__ void __launch_bounds__(128, kMinBlocks)
     const int lanes = P.lanes_per_azimuth;
     const int azimuths_per_job = 32 / lanes;
     unsigned visits = 0, samples = 0, steps = 0;
-    __shared__ typename std::conditional<kLadder == kReference, RayStore::Block, char>::type store;
+    __shared__ typename std::conditional<kLadder == kReference, SitesBlock, char>::type
+        store;
     for (;;) {
         unsigned long long taken = 0;
         if (lane == 0) taken = atomicAdd(P.next_job, 1ull);
@@ -131,6 +155,14 @@ __global__ void __launch_bounds__(128, kMinBlocks)
         const bool in_tile = azimuth < P.azimuth_count;
         const bool marches = in_tile && tile.tile_column + column < primary_width &&
                              tile.tile_row + row < primary_height;
+        if constexpr ((kLadder & kRelative) != 0) {
+            // No warp-wide step below: a lane without a ray goes to the next job.
+            if (!in_tile) continue;
+            if (!marches) {
+                *out = -INFINITY;
+                continue;
+            }
+        }
         float observer_z = 0.0f, current = -1e30f;
         if (marches)
             observer_z = __fadd_rn(
@@ -150,15 +182,31 @@ __global__ void __launch_bounds__(128, kMinBlocks)
                     primary_height, ratio);
             }
             if constexpr (kArgmax) tracker.current_pass = d;
-            const GlobalLevels levels{&dem.table};
-            if constexpr (kLadder == kReference)
+            if constexpr (kLadder != kReference) {
+                if (marches)
+                    current = march_dem_tracked<kCount, kLadder>(GlobalLevels{&dem.table}, view, g,
+                                                                 d, observer_z, current, visits,
+                                                                 samples, steps, tracker);
+            } else {
+                // The warp's own copy of the DEM's level table.
+                WarpDem &here = store.dems[threadIdx.x >> 5];
+                __syncwarp();
+                if (lane == 0)
+                    here.last = make_float2(static_cast<float>(view.width - 1),
+                                            static_cast<float>(view.height - 1));
+                if (lane < view.level_count) {
+                    here.table.side[lane] = __ldg(&dem.table.side[lane]);
+                    here.table.fallback[lane] = __ldg(&dem.table.fallback[lane]);
+                    here.table.out_step[lane] = __ldg(&dem.table.out_step[lane]);
+                    here.table.cells[lane] = __ldg(&dem.table.cells[lane]);
+                }
+                __syncwarp();
+                const WarpLevels levels{here.table, here.last};
+                const RayStore rays(store.rays);
                 current = march_dem_far<kCount, false>(levels, view, g, d, observer_z, current,
-                                                       marches, RayStore(store), visits, samples,
-                                                       steps, tracker);
-            else if (marches)
-                current = march_dem_tracked<kCount, kLadder>(levels, view, g, d, observer_z,
-                                                             current, visits, samples, steps,
-                                                             tracker);
+                                                       marches, rays, visits, samples, steps,
+                                                       tracker);
+            }
         }
         if (!in_tile) continue;
         if constexpr (kArgmax) {
@@ -192,7 +240,11 @@ static void dispatch(ls200_context *ctx, const SitesParams &P, int traversal) {
     switch (traversal) {
         case kReference: launch_sites<kCount, kReference, kMinBlocks>(ctx, P); break;
         case kLadderClimb: launch_sites<kCount, kLadderClimb, kMinBlocks>(ctx, P); break;
-        case kRelative: launch_sites<kCount, kRelative, kMinBlocks>(ctx, P); break;
+        case kRelative:
+            // 64 registers spill too much here: 349.6 ms at 7 blocks for two
+            // sites of 2048^2 over 3072^2, 353.4 at 8.
+            launch_sites<kCount, kRelative, (kMinBlocks > 7 ? 7 : kMinBlocks)>(ctx, P);
+            break;
         default: launch_sites<kCount, kLadderClimb | kRelative, kMinBlocks>(ctx, P); break;
     }
 }

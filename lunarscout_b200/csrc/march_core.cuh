@@ -38,7 +38,8 @@
 //     the reference arithmetic inside it (bound_culled);
 //   * in the reference traversal most far-field culls are settled by a step
 //     of 55 instructions that computes exactly only what moves the ray
-//     (FarRay, march_dem_far), and most other steps by level0_step.
+//     (FarRay, march_dem_far), most other steps by level0_step, and the
+//     first 500 m of a ray by march_near.
 //
 // The skip ladder (kLadder, the batched traversal; no reference counterpart)
 // extends a cull to the largest culled ancestor cell, see ladder_advance.
@@ -823,21 +824,30 @@ struct FarRange {
     float end;  // steps may settle from 500 m up to here (km; -inf: none)
 };
 
+__device__ __forceinline__ float path_reach(const RaySegment &g) {
+    const float span = g.s_end - g.s_start;
+    return span * (fabsf(g.k1.x) + fabsf(g.k1.y) +
+                   span * (fabsf(g.k2.x) + fabsf(g.k2.y) +
+                           span * (fabsf(g.k3.x) + fabsf(g.k3.y) +
+                                   span * (fabsf(g.k4.x) + fabsf(g.k4.y)))));
+}
+
+__device__ __forceinline__ bool far_tame(const DemView &dem, const RaySegment &g,
+                                         float observer_z) {
+    const float reach = path_reach(g);
+    const float planar = reach * dem.resolution * 1.0001f;
+    return g.s_end - g.s_start >= 1e-3f && reach < 4e6f && fabsf(g.start.x) < 4e6f &&
+           fabsf(g.start.y) < 4e6f && g.s_start_chord >= 0.0f && g.s_start_chord < 1e6f &&
+           g.c1 >= 0.1f && g.c1 <= 10.0f &&
+           planar * (fabsf(g.c2) + planar * fabsf(g.c3)) <= 0.2f * g.c1 &&
+           dem.width <= (1 << 22) && dem.height <= (1 << 22) && fabsf(observer_z) < 1e6f &&
+           dem.radius > 1e5f && dem.radius < 1e9f;
+}
+
 __device__ __forceinline__ FarRange far_range(const DemView &dem, const RaySegment &g,
                                               float observer_z) {
-    const float span = g.s_end - g.s_start;
-    const float reach =
-        span * (fabsf(g.k1.x) + fabsf(g.k1.y) +
-                span * (fabsf(g.k2.x) + fabsf(g.k2.y) +
-                        span * (fabsf(g.k3.x) + fabsf(g.k3.y) +
-                                span * (fabsf(g.k4.x) + fabsf(g.k4.y)))));
-    const float planar = reach * dem.resolution * 1.0001f;
-    const bool tame = span >= 1e-3f && reach < 4e6f && fabsf(g.start.x) < 4e6f &&
-                      fabsf(g.start.y) < 4e6f && g.s_start_chord >= 0.0f &&
-                      g.s_start_chord < 1e6f && g.c1 >= 0.1f && g.c1 <= 10.0f &&
-                      planar * (fabsf(g.c2) + planar * fabsf(g.c3)) <= 0.2f * g.c1 &&
-                      dem.width <= (1 << 22) && dem.height <= (1 << 22) &&
-                      fabsf(observer_z) < 1e6f && dem.radius > 1e5f && dem.radius < 1e9f;
+    const float span = g.s_end - g.s_start, reach = path_reach(g);
+    const bool tame = far_tame(dem, g, observer_z);
     const float a = fmaxf(0.5f - g.s_start, 0.0f);
     const float2 a2 = pair(a, a);
     const float2 t0 = __ffma2_rn(a2, __ffma2_rn(a2, __ffma2_rn(a2, __ffma2_rn(a2, g.k4, g.k3),
@@ -931,10 +941,62 @@ __device__ __forceinline__ float chord_distance_m(const RaySegment &g, float2 r,
     return __fmaf_rn(g.s_start_chord, 1000.0f, chord);
 }
 
+// The level-0 sample of a step, in the reference's arithmetic: its slope, the
+// running maximum and the advance.  q.. are the cell's corners, `corner` its
+// integer position; which of pixel, angular and floor step is the largest is
+// decided by a bound where that is clear.
+template <class Tracker>
+__device__ __forceinline__ void sample_step(const DemView &dem, int pass_index, float observer_z,
+                                            float observer_radius, bool near, float2 p,
+                                            float2 corner, float2 tangent, float true_m,
+                                            float q00, float q10, float q01, float q11,
+                                            MarchState &st, Tracker &tracker) {
+    const float current = st.current, resolution = dem.resolution;
+    const bool valid = q00 > -20000.0f && q10 > -20000.0f && q01 > -20000.0f && q11 > -20000.0f;
+    const float2 t = sub2(p, corner);
+    const float top = __fmaf_rn(t.x, __fsub_rn(q10, q00), q00);
+    const float bottom = __fmaf_rn(t.x, __fsub_rn(q11, q01), q01);
+    const float height = __fmaf_rn(t.y, __fsub_rn(bottom, top), top);
+    float slope = -1e30f;
+    if (valid) {
+        slope = near ? __fdiv_rn(__fsub_rn(height, observer_z), true_m)
+                     : sample_slope(true_m, height, dem.radius, observer_radius);
+        if (slope > current) {
+            st.current = slope;
+            tracker.record(p.x, p.y, true_m, slope, near);
+        }
+    }
+    // The smaller of the margin's and the angular product, over 1000 (see
+    // march_step).
+    const float angular = __fmul_rn(true_m, 0.00151f);
+    const float margin = __fsub_rn(st.current, slope);
+    float product = 0.0f;
+    if (margin > 0.0f) {
+        const float margin_product = __fmul_rn(__fmul_rn(margin, true_m), 1.732f);
+        product = margin_product < angular ? margin_product : angular;
+    }
+    const float floor_step = pass_index == 0 && true_m >= 100.0f
+                                 ? __fmul_rn(__fmul_rn(0.8f, resolution), 0.001f)
+                                 : __fmul_rn(__fmul_rn(0.5f, resolution), 0.001f);
+    const float scale = near ? 0.25f : 1.0f;
+    float advance = over_1000(product);
+    const float squared = tangent.x * tangent.x + tangent.y * tangent.y;
+    const float pixel_most = rsqrtf(squared) * 1.00001f;
+    if (!(squared > 1e-11f) ||
+        !(advance > pixel_most || pixel_most * scale < floor_step * 0.99999f)) {
+        const float magnitude = hypot_fused(tangent.x, tangent.y);
+        const float pixel_step = magnitude > 1e-6f ? __frcp_rn(magnitude) : 0.0005f;
+        advance = pixel_step > advance ? pixel_step : advance;
+    }
+    advance = __fmul_rn(advance, scale);
+    advance = advance > floor_step ? advance : floor_step;
+    st.s = __fadd_rn(st.s, advance);
+}
+
 // One step at level 0 in the reference's arithmetic, for the rays far_range
 // found tame and positions whose clamps do not act: most steps that far_step
-// leaves over, in the near field all.  Returns false, having done nothing,
-// when the step is another one.  The cull (one product per side) and which
+// leaves over.  Returns false, having done nothing, when the step is another
+// one.  The cull (one product per side) and which
 // of pixel, angular and floor step is the largest are again decided by a
 // bound on the error where that is clear.
 template <bool kCount, bool kAhead, class Table, class Tracker>
@@ -1010,45 +1072,8 @@ __device__ __forceinline__ bool level0_step(const Table &table, const DemView &d
         q00 = __ldg(r0), q10 = __ldg(r0 + 1);
         q01 = __ldg(r1), q11 = __ldg(r1 + 1);
     }
-    const bool valid = q00 > -20000.0f && q10 > -20000.0f && q01 > -20000.0f && q11 > -20000.0f;
-    const float2 t = sub2(p, corner);
-    const float top = __fmaf_rn(t.x, __fsub_rn(q10, q00), q00);
-    const float bottom = __fmaf_rn(t.x, __fsub_rn(q11, q01), q01);
-    const float height = __fmaf_rn(t.y, __fsub_rn(bottom, top), top);
-    float slope = -1e30f;
-    if (valid) {
-        slope = near ? __fdiv_rn(__fsub_rn(height, observer_z), true_m)
-                     : sample_slope(true_m, height, dem.radius, observer_radius);
-        if (slope > current) {
-            st.current = slope;
-            tracker.record(p.x, p.y, true_m, slope, near);
-        }
-    }
-    // The smaller of the margin's and the angular product, over 1000 (see
-    // march_step).
-    const float angular = __fmul_rn(true_m, 0.00151f);
-    const float margin = __fsub_rn(st.current, slope);
-    float product = 0.0f;
-    if (margin > 0.0f) {
-        const float margin_product = __fmul_rn(__fmul_rn(margin, true_m), 1.732f);
-        product = margin_product < angular ? margin_product : angular;
-    }
-    const float floor_step = pass_index == 0 && true_m >= 100.0f
-                                 ? __fmul_rn(__fmul_rn(0.8f, resolution), 0.001f)
-                                 : __fmul_rn(__fmul_rn(0.5f, resolution), 0.001f);
-    const float scale = near ? 0.25f : 1.0f;
-    float advance = over_1000(product);
-    const float squared = tangent.x * tangent.x + tangent.y * tangent.y;
-    const float pixel_most = rsqrtf(squared) * 1.00001f;
-    if (!(squared > 1e-11f) ||
-        !(advance > pixel_most || pixel_most * scale < floor_step * 0.99999f)) {
-        const float magnitude = hypot_fused(tangent.x, tangent.y);
-        const float pixel_step = magnitude > 1e-6f ? __frcp_rn(magnitude) : 0.0005f;
-        advance = pixel_step > advance ? pixel_step : advance;
-    }
-    advance = __fmul_rn(advance, scale);
-    advance = advance > floor_step ? advance : floor_step;
-    st.s = __fadd_rn(s, advance);
+    sample_step(dem, pass_index, observer_z, observer_radius, near, p, corner, tangent, true_m,
+                q00, q10, q01, q11, st, tracker);
     return true;
 }
 
@@ -1235,6 +1260,105 @@ __device__ __forceinline__ float march_dem_tracked(const Table &table, const Dem
     return st.current;
 }
 
+// The near field (the first 500 m) of one ray: at level 0 throughout, and its
+// samples advance by the floor step whatever the slope, because a quarter of a
+// pixel's step and of the angular step stay below it (checked for the segment).
+// So a sample needs its slope only when it may raise the maximum, and a step
+// needs the tangent only when its cell is culled: 60 instructions where
+// level0_step takes 200 (a site-scale tile 183 -> 174.5 ms, a preview tile of
+// 20 km rays 265 -> 252 us).  A ray meets a step it does not cover (the DEM's edge,
+// an axis-parallel exit) by leaving; the caller's loop goes on from there.
+// Returns the path position reached; every lane of the warp calls it.
+template <bool kCount, class Table, class Tracker>
+__device__ __forceinline__ float march_near(const Table &table, const DemView &dem,
+                                            const RaySegment &g, bool tame, int pass_index,
+                                            float observer_z, float s, float &current,
+                                            unsigned &visits, unsigned &samples,
+                                            unsigned &steps, Tracker &tracker) {
+    const float resolution = dem.resolution;
+    const float floor_step = __fmul_rn(__fmul_rn(0.5f, resolution), 0.001f);
+    const float far_floor = pass_index == 0
+                                ? __fmul_rn(__fmul_rn(0.8f, resolution), 0.001f) : floor_step;
+    // The tangent's least length over the near field, in pixels per km.
+    const float bend = (fabsf(g.k2.x) + fabsf(g.k2.y)) +
+                       0.75f * (fabsf(g.k3.x) + fabsf(g.k3.y)) +
+                       0.5f * (fabsf(g.k4.x) + fabsf(g.k4.y));
+    const float least = 0.9999f * sqrt_approx(g.k1.x * g.k1.x + g.k1.y * g.k1.y) - bend;
+    const bool covered = tame && least * floor_step > 0.2501f && floor_step > 1.89e-4f &&
+                         (dem.level_count < 2 || table.side(1) > 2.2f);
+    const float xmax = fminf(static_cast<float>(dem.width) - 1.0001f,
+                             static_cast<float>(dem.width - 1) - 0.5f);
+    const float ymax = fminf(static_cast<float>(dem.height) - 1.0001f,
+                             static_cast<float>(dem.height - 1) - 0.5f);
+    bool live = covered && s < 0.5f && s <= g.s_end;
+    while (__any_sync(0xffffffffu, live)) {
+        if (live) {
+            const float delta = __fsub_rn(s, g.s_start);
+            const float2 d1 = pair(delta, delta);
+            const float2 d2 = __fmul2_rn(d1, d1);
+            const float2 d3 = __fmul2_rn(d2, d1);
+            const float2 d4 = __fmul2_rn(d2, d2);
+            const float2 p = quartic2(g.start, g.k1, g.k2, g.k3, g.k4, d1, d2, d3, d4);
+            live = p.x >= 0.0f && p.y >= 0.0f && p.x < xmax && p.y < ymax;
+            if (live) {
+                const float true_m = __fmul_rn(s, 1000.0f);
+                const float2 down = add2_down(p, pair(0x1p23f, 0x1p23f));
+                const float2 corner = __fadd2_rn(down, pair(-0x1p23f, -0x1p23f));
+                const int index = (__float_as_int(down.y) - 0x4b000000) * dem.width +
+                                  (__float_as_int(down.x) - 0x4b000000);
+                const float *r0 = dem.cells + index, *r1 = r0 + dem.width;
+                const float maximum_height = __ldg(dem.bounds + index);
+                const float q00 = __ldg(r0), q10 = __ldg(r0 + 1);
+                const float q01 = __ldg(r1), q11 = __ldg(r1 + 1);
+                const float dh = __fsub_rn(maximum_height, observer_z);
+                float true_near = __fsub_rn(true_m, resolution);
+                true_near = true_near > 1.0f ? true_near : 1.0f;
+                const float limit = current * true_near;
+                const float band = 1e-5f * fabsf(limit) + 1e-30f;
+                bool culled = maximum_height < -20000.0f || dh < limit - band;
+                if (!culled && !(dh > limit + band)) culled = __fdiv_rn(dh, true_near) <= current;
+                if (culled) {
+                    const float2 tangent = quartic_tangent2(g.k1, g.k2, g.k3, g.k4, d1, d2, d3);
+                    if (fabsf(tangent.x) > 1e-8f && fabsf(tangent.y) > 1e-8f) {
+                        const float2 edge =
+                            __fadd2_rn(corner, pair(tangent.x > 0.0f ? 1.0f : 0.0f,
+                                                    tangent.y > 0.0f ? 1.0f : 0.0f));
+                        const float2 exits = __fmul2_rn(sub2(p, edge),
+                                                        newton_minus_reciprocal_pair(tangent));
+                        const float exit = fminf(exits.x, exits.y);
+                        s = __fadd_rn(s, __fadd_rn(exit > 0.0f ? exit : table.fallback(0),
+                                                   0.0001f));
+                        if (kCount) ++steps, ++visits;
+                    } else {
+                        live = false;
+                    }
+                } else {
+                    if (q00 > -20000.0f && q10 > -20000.0f && q01 > -20000.0f &&
+                        q11 > -20000.0f) {
+                        const float2 t = sub2(p, corner);
+                        const float top = __fmaf_rn(t.x, __fsub_rn(q10, q00), q00);
+                        const float bottom = __fmaf_rn(t.x, __fsub_rn(q11, q01), q01);
+                        const float height = __fmaf_rn(t.y, __fsub_rn(bottom, top), top);
+                        const float rise = __fsub_rn(height, observer_z);
+                        const float least_rise = current * true_m;
+                        if (!(rise < least_rise - 1e-6f * fabsf(least_rise))) {
+                            const float slope = __fdiv_rn(rise, true_m);
+                            if (slope > current) {
+                                current = slope;
+                                tracker.record(p.x, p.y, true_m, slope, true);
+                            }
+                        }
+                    }
+                    s = __fadd_rn(s, true_m >= 100.0f ? far_floor : floor_step);
+                    if (kCount) ++steps, ++visits, ++samples;
+                }
+                live = live && s < 0.5f && s <= g.s_end;
+            }
+        }
+    }
+    return s;
+}
+
 // The step of a lane that far_step left over: level0_step or the reference's
 // full step, and what they change for the next fast steps.
 template <bool kCount, bool kAhead, class Table, class Tracker>
@@ -1282,12 +1406,7 @@ __device__ __forceinline__ void slow_step(FarCell &far, const RayStore &store, c
 // ray.  The fast step has no branch; the lanes it leaves over step together.
 // The votes also keep the warp together: without one per step the settled
 // lanes ran ahead while the others waited (4.3 times slower).
-// kNearFirst marches the near field, where no step settles, in a loop of its
-// own and loads corners ahead, which shortens a launch of few warps (the
-// 16 x 16 x 72 ray preview 282 -> 265 us, the site-scale tile 185.3 -> 183.3
-// ms); the persistent kernel, already out of registers, does without (212
-// instead of 221 ms on two sites).
-template <bool kCount, bool kNearFirst, class Table, class Tracker>
+template <bool kCount, bool kAhead, class Table, class Tracker>
 __device__ __forceinline__ float march_dem_far(const Table &table, const DemView &dem,
                                                const RaySegment &g, int pass_index,
                                                float observer_z, float current, bool marches,
@@ -1297,7 +1416,9 @@ __device__ __forceinline__ float march_dem_far(const Table &table, const DemView
     const MarchState first = begin_pass(dem, g, current);
     const FarRange range = far_range(dem, g, observer_z);
     // A lane whose ray has ended (or never was) stands at +inf.
-    float s = marches ? first.s : INFINITY;
+    float s = march_near<kCount>(table, dem, g, range.tame, pass_index, observer_z,
+                                 marches ? first.s : INFINITY, current, visits, samples, steps,
+                                 tracker);
     const float height_base = observer_z - 5e-6f * (32768.0f + fabsf(observer_z));
     const float double_radius = 2.0f * (dem.radius + observer_z) * 1.000004f;
     FarCell far;
@@ -1305,7 +1426,7 @@ __device__ __forceinline__ float march_dem_far(const Table &table, const DemView
     far_ahead(far, pair(-1.0f, -1.0f));
     store.save(0, s >= 0.5f ? range.end : -INFINITY, height_base, double_radius,
                far_sine(dem.radius + observer_z, current));
-    store.set(RayStore::kCurrent, first.current);
+    store.set(RayStore::kCurrent, current);
     store.set(RayStore::kSideUp, first.side_up);
     store.set(RayStore::kSideHere, first.side_here);
     store.set(RayStore::kLevel, __int_as_float(first.level_hint));
@@ -1313,18 +1434,6 @@ __device__ __forceinline__ float march_dem_far(const Table &table, const DemView
     store.set(RayStore::kChord, g.s_start_chord);
     store.set(RayStore::kObserver, observer_z);
     store.set(RayStore::kLimit, range.tame ? range.end : INFINITY);  // +inf: not tame
-    // The near field: every step is a full one.
-    bool near = kNearFirst && s < 0.5f;
-    while (kNearFirst && __any_sync(0xffffffffu, near)) {
-        const float s_end = store.get(RayStore::kEnd);
-        if (near && !(s <= s_end)) s = INFINITY;
-        else if (near) {
-            const StepPoint at = step_point<false>(g, s);
-            slow_step<kCount, true>(far, store, table, dem, g, at, pass_index, s_end, s,
-                                    visits, samples, steps, tracker);
-        }
-        near = s < 0.5f;
-    }
     for (;;) {
         const StepPoint at = step_point<false>(g, s);
         const bool settled = far_step(far, store, dem, g, at.p, at.minus_inv, s);
@@ -1332,8 +1441,8 @@ __device__ __forceinline__ float march_dem_far(const Table &table, const DemView
         if (__any_sync(0xffffffffu, !settled)) {
             const float s_end = store.get(RayStore::kEnd);
             if (!settled && s <= s_end)
-                slow_step<kCount, kNearFirst>(far, store, table, dem, g, at, pass_index, s_end, s,
-                                              visits, samples, steps, tracker);
+                slow_step<kCount, kAhead>(far, store, table, dem, g, at, pass_index, s_end, s,
+                                          visits, samples, steps, tracker);
             if (!__any_sync(0xffffffffu, s <= s_end)) break;
         }
     }

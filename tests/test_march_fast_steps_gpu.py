@@ -90,3 +90,49 @@ def test_settled_steps_keep_every_slope_and_decision(name, cuda_session):
     np.testing.assert_array_equal(gpu, cpu)
     np.testing.assert_array_equal(counted, cpu)
     assert (visits, samples) == tuple(expected)
+
+
+@pytest.mark.parametrize("traversal", ["exact", "ladder"])
+@pytest.mark.parametrize("name", ["axis", "coarse", "corner", "far edge", "few cells", "fine",
+                                  "invalid", "two passes", "walls"])
+def test_batched_settled_steps_keep_every_slope_and_decision(name, traversal, cuda_session):
+    """The persistent march's steps (march_near among them) on the
+    same DEMs: whole tiles of 12 azimuths against the oracle's restatement."""
+    import torch
+
+    from lunarscout_b200.contract import PyramidArrays, map_parameters, projection_parameters
+    from lunarscout_b200.cuda_backend import SiteTile
+
+    dems, column, row, _, _, _, distance = CASES[name]()
+    azimuths = 12
+    device = [cuda_session.upload_dem_grid(dem) for dem in dems]
+    tile = SiteTile(tuple(device), column, row, distance, 2.0)
+    out = torch.empty(128 * 128 * azimuths, device="cuda")
+    torch.cuda.synchronize()
+    cuda_session.march_sites([tile], device_out=out.data_ptr(), azimuth_count=azimuths,
+                             traversal=traversal)
+    plain = out.cpu().numpy().reshape(128 * 128, azimuths)
+    cuda_session.set_counting(True)
+    try:
+        cuda_session.march_sites([tile], device_out=out.data_ptr(), azimuth_count=azimuths,
+                                 traversal=traversal)
+        visits, samples, _ = cuda_session.last_counters()
+    finally:
+        cuda_session.set_counting(False)
+    pyramids = []
+    for dem in dems:
+        mips, levels = oracle.build_pyramid(dem.elevation_m)
+        pyramids.append(PyramidArrays(dem.elevation_m, mips, levels, map_parameters(dem),
+                                      projection_parameters(dem)))
+    segments = cuda_session.generate_segments(
+        device, tile_column=column, tile_row=row, azimuth_count=azimuths,
+        maximum_distance_m=distance, observer_elevation_m=2.0)
+    mask = oracle.ladder_mask(0, 1) if traversal == "ladder" else oracle.PRODUCTION_MASK
+    expected, counts = oracle.march_all_passes(
+        segments, pyramids, tile_column=column, tile_row=row, observer_elevation_m=2.0,
+        mask=mask)
+    np.testing.assert_array_equal(plain, expected)
+    np.testing.assert_array_equal(out.cpu().numpy().reshape(expected.shape), expected)
+    assert (visits, samples) == tuple(counts)
+    for dem in device:
+        dem.close()
