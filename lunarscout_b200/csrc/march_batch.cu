@@ -15,7 +15,9 @@
 // a cull climbs to the largest culled ancestor cell, which removes most of
 // the footprint-limited steps of long rays; its results are checked against
 // its own CPU restatement (oracle flag OPT_LADDER) and their distance from
-// the FP64 restatement is measured beside the reference traversal's.
+// the FP64 restatement is measured beside the reference traversal's.  Its far
+// field runs warp-wide with the culls settled by their bounds (march_dem_ladder:
+// eight sites 430 -> 390 ms).
 //
 // Launch configuration (autotuned, never changing results): how the 32 lanes
 // of a job map onto rays (L adjacent pixels x 32/L adjacent azimuths, L a
@@ -73,7 +75,7 @@ struct SitesParams {
 };
 
 // Level table read through the read-only path (each warp may be on a
-// different DEM; the tables stay resident in L1).
+// different DEM; the tables stay resident in L1): the relative traversals.
 struct GlobalLevels {
     const LevelTable *t;
     __device__ __forceinline__ float side(int l) const { return __ldg(&t->side[l]); }
@@ -131,7 +133,7 @@ __global__ void __launch_bounds__(128, kMinBlocks)
     const int lanes = P.lanes_per_azimuth;
     const int azimuths_per_job = 32 / lanes;
     unsigned visits = 0, samples = 0, steps = 0;
-    __shared__ typename std::conditional<kLadder == kReference, SitesBlock, char>::type
+    __shared__ typename std::conditional<(kLadder & kRelative) == 0, SitesBlock, char>::type
         store;
     for (;;) {
         unsigned long long taken = 0;
@@ -182,11 +184,10 @@ __global__ void __launch_bounds__(128, kMinBlocks)
                     primary_height, ratio);
             }
             if constexpr (kArgmax) tracker.current_pass = d;
-            if constexpr (kLadder != kReference) {
-                if (marches)
-                    current = march_dem_tracked<kCount, kLadder>(GlobalLevels{&dem.table}, view, g,
-                                                                 d, observer_z, current, visits,
-                                                                 samples, steps, tracker);
+            if constexpr ((kLadder & kRelative) != 0) {
+                current = march_dem_tracked<kCount, kLadder>(GlobalLevels{&dem.table}, view, g, d,
+                                                             observer_z, current, visits, samples,
+                                                             steps, tracker);
             } else {
                 // The warp's own copy of the DEM's level table.
                 WarpDem &here = store.dems[threadIdx.x >> 5];
@@ -203,9 +204,14 @@ __global__ void __launch_bounds__(128, kMinBlocks)
                 __syncwarp();
                 const WarpLevels levels{here.table, here.last};
                 const RayStore rays(store.rays);
-                current = march_dem_far<kCount, false>(levels, view, g, d, observer_z, current,
+                if constexpr (kLadder == kLadderClimb)
+                    current = march_dem_ladder<kCount>(levels, view, g, d, observer_z, current,
                                                        marches, rays, visits, samples, steps,
                                                        tracker);
+                else
+                    current = march_dem_far<kCount, false>(levels, view, g, d, observer_z,
+                                                           current, marches, rays, visits,
+                                                           samples, steps, tracker);
             }
         }
         if (!in_tile) continue;
@@ -249,13 +255,12 @@ static void dispatch(ls200_context *ctx, const SitesParams &P, int traversal) {
     }
 }
 
-// The checkpointing march runs 8 blocks per SM too: its extra tracker
-// registers spill a little at 64, which costs less than the occupancy of 6
-// blocks at 80 registers (measured: the differentiable workload's forward
-// 294 -> 267 ms, the 8192^2 slice's 2.58 -> 2.04 s).
+// The checkpointing march runs 7 blocks per SM (72 registers): its tracker
+// spills more at 64 (the differentiable workload's forward and backward pass,
+// one tile: 50 ms, 51 at 8).
 static void dispatch_argmax(ls200_context *ctx, const SitesParams &P, int traversal) {
-    if (traversal == kReference) launch_sites<false, kReference, 8, true>(ctx, P);
-    else launch_sites<false, kLadderClimb, 8, true>(ctx, P);
+    if (traversal == kReference) launch_sites<false, kReference, 7, true>(ctx, P);
+    else launch_sites<false, kLadderClimb, 7, true>(ctx, P);
 }
 
 static size_t align_up(size_t n) { return (n + 255) & ~size_t(255); }

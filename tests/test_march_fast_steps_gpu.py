@@ -96,7 +96,7 @@ def test_settled_steps_keep_every_slope_and_decision(name, cuda_session):
 @pytest.mark.parametrize("name", ["axis", "coarse", "corner", "far edge", "few cells", "fine",
                                   "invalid", "two passes", "walls"])
 def test_batched_settled_steps_keep_every_slope_and_decision(name, traversal, cuda_session):
-    """The persistent march's steps (march_near among them) on the
+    """The persistent march's steps (ladder_step, march_near among them) on the
     same DEMs: whole tiles of 12 azimuths against the oracle's restatement."""
     import torch
 
