@@ -1026,6 +1026,11 @@ void mission_duration_launch(ls200_context *ctx, LightingBatch &B, int tiles,
 // hours = float32(longest) * float32(time_step_hours), NaN where the band saw
 // no outage or nothing else (safe_haven.py:231-240) and outside the valid
 // rectangle.
+//
+// The bits are taken a word at a time: the warp splits a word where the month
+// changes (the months are the same for every pixel), and within a part only
+// the ends of low-Sun runs are visited.  One step at a time was a chain of 25
+// instructions for each sample of a pixel.
 struct HavenParams {
     const uint32_t *low, *outage;  // [tiles, words, 16384]
     const int *month;              // [T] band of each time step, -1 for none
@@ -1049,11 +1054,14 @@ __global__ void __launch_bounds__(128) haven_kernel(const __grid_constant__ Have
     const bool valid = index % kPatch < P.valid[tile].x && index / kPatch < P.valid[tile].y;
     if (!valid) {
         for (int b = 0; b < P.bands; ++b) out[b * plane] = __int_as_float(0x7fffffff);
-        return;
     }
-    for (int b = 0; b < P.bands; ++b) {
-        longest[b * plane] = 0;
-        flags[b * plane] = 0;
+    // The other lanes of the warp stay for the votes on the months.
+    if (!__any_sync(0xffffffffu, valid)) return;
+    if (valid) {
+        for (int b = 0; b < P.bands; ++b) {
+            longest[b * plane] = 0;
+            flags[b * plane] = 0;
+        }
     }
     int run = 0;
     int lo = P.bands, hi = -1;       // bands the current run touched lie in [lo, hi]
@@ -1075,35 +1083,70 @@ __global__ void __launch_bounds__(128) haven_kernel(const __grid_constant__ Have
         lo = P.bands;
         hi = -1;
     };
-    const size_t word0 = static_cast<size_t>(tile) * P.words * plane + index;
-    for (int w = 0; w < P.words; ++w) {
-        const uint32_t low_word = __ldg(P.low + word0 + w * plane);
-        const uint32_t outage_word = __ldg(P.outage + word0 + w * plane);
-        const int steps = min(32, P.time_count - w * 32);
-        for (int j = 0; j < steps; ++j) {
-            const bool low = (low_word >> j) & 1u;
-            const bool outage = (outage_word >> j) & 1u;
-            if (low) {
-                ++run;
-            } else {
-                if (hi >= 0) credit();
-                run = 0;
+    // Samples [first, last) of a word, all of month m.
+    auto part = [&](uint32_t low_word, uint32_t outage_word, int first, int last, int m) {
+        const uint32_t mask = (0xffffffffu >> (32 - last)) & (0xffffffffu << first);
+        const uint32_t high = ~low_word & mask;
+        uint32_t touches = 0u;  // samples that credit their run to the band
+        if (m >= 0) {
+            if (m != cached) {
+                store();
+                cached = m;
             }
-            const int m = __ldg(P.month + w * 32 + j);
-            if (m >= 0) {
-                if (m != cached) {
-                    store();
-                    cached = m;
-                }
-                bits |= outage ? 1u : 2u;
-                if (outage && low) {
-                    bits |= 4u;
-                    lo = min(lo, m);
-                    hi = max(hi, m);
-                }
+            bits |= ((outage_word & mask) ? 1u : 0u) | ((~outage_word & mask) ? 2u : 0u);
+            touches = low_word & outage_word & mask;
+        }
+        auto touch = [&](uint32_t run_mask) {
+            if (touches & run_mask) {
+                bits |= 4u;
+                lo = min(lo, m);
+                hi = max(hi, m);
+            }
+        };
+        int from = first;  // every sample of the part below it is done
+        uint32_t left = high;
+        while (left) {
+            const int end = __ffs(left) - 1;  // the run, if any, is [.., end)
+            run += end - from;
+            touch((1u << end) - (1u << from));
+            if (hi >= 0) credit();
+            run = 0;
+            const uint32_t lows = low_word & mask & (0xffffffffu << end);
+            if (!lows) return;
+            from = __ffs(lows) - 1;
+            left = high & (0xffffffffu << from);
+        }
+        run += last - from;
+        touch(mask & (0xffffffffu << from));
+    };
+    const int lane = threadIdx.x & 31;
+    const size_t word0 = static_cast<size_t>(tile) * P.words * plane + index;
+    constexpr int kAhead = 4;  // words loaded together
+    for (int w0 = 0; w0 < P.words; w0 += kAhead) {
+        uint32_t low_words[kAhead], outage_words[kAhead];
+        int months[kAhead];
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) {
+            const int w = min(w0 + j, P.words - 1);
+            low_words[j] = __ldg(P.low + word0 + w * plane);
+            outage_words[j] = __ldg(P.outage + word0 + w * plane);
+            months[j] = __ldg(P.month + min(w * 32 + lane, P.time_count - 1));
+        }
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) {
+            if (w0 + j >= P.words) break;
+            const int steps = min(32, P.time_count - (w0 + j) * 32);
+            for (int first = 0; first < steps;) {
+                const int m = __shfl_sync(0xffffffffu, months[j], first);
+                const uint32_t others =
+                    __ballot_sync(0xffffffffu, months[j] != m) & (0xffffffffu << first);
+                const int last = others ? min(__ffs(others) - 1, steps) : steps;
+                if (valid) part(low_words[j], outage_words[j], first, last, m);
+                first = last;
             }
         }
     }
+    if (!valid) return;
     if (hi >= 0) credit();  // the run still open at the end is right-censored
     store();
     for (int b = 0; b < P.bands; ++b) {
