@@ -660,10 +660,68 @@ int lighting_chunk(ls200_context *ctx, int tiles, int time_count) {
     return (time_count + chunks - 1) / chunks;
 }
 
+// The time indices of a table in longitude order, to a bin of 0.044 degrees (a
+// sixth of a horizon bin: what the staged windows gain is the neighbourhood,
+// and outputs do not depend on the order).  A counting sort in one block, the
+// bins of the steps kept in `scratch` [count]; non-finite longitudes count as
+// 0.  Creating and closing a table took a sort by atan2 on the host: 31 us for
+// 125 vectors, 231 for 8,761, 677 for 26,281; now 28, 46 and 76.
+constexpr int kOrderThreads = 1024;
+constexpr int kOrderBins = 8192;
+
+__global__ void __launch_bounds__(kOrderThreads) longitude_order_kernel(
+    const float *__restrict__ vectors, int count, int *__restrict__ scratch,
+    int *__restrict__ order) {
+    constexpr int kPer = kOrderBins / kOrderThreads;
+    __shared__ int bins[kOrderBins];
+    __shared__ int warp_sums[32];
+    for (int b = threadIdx.x; b < kOrderBins; b += kOrderThreads) bins[b] = 0;
+    __syncthreads();
+    for (int t = threadIdx.x; t < count; t += kOrderThreads) {
+        const float *v = vectors + 3 * static_cast<size_t>(t);
+        const float longitude = atan2f(v[1], v[0]);
+        const float scaled =
+            (isfinite(longitude) ? longitude : 0.0f) * (kOrderBins / 6.2831855f) + kOrderBins / 2;
+        const int bin = min(max(static_cast<int>(scaled), 0), kOrderBins - 1);
+        scratch[t] = bin;
+        atomicAdd(&bins[bin], 1);
+    }
+    __syncthreads();
+    // Exclusive sums: the thread's own bins, its warp, the block.
+    const int lane = threadIdx.x & 31;
+    int mine = 0;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) mine += bins[threadIdx.x * kPer + j];
+    int sum = mine;
+#pragma unroll
+    for (int offset = 1; offset < 32; offset <<= 1) {
+        const int add = __shfl_up_sync(0xffffffffu, sum, offset);
+        if (lane >= offset) sum += add;
+    }
+    if (lane == 31) warp_sums[threadIdx.x >> 5] = sum;
+    __syncthreads();
+    int position = sum - mine;
+    for (int w = 0; w < static_cast<int>(threadIdx.x >> 5); ++w) position += warp_sums[w];
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        const int n = bins[threadIdx.x * kPer + j];
+        bins[threadIdx.x * kPer + j] = position;
+        position += n;
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < count; t += kOrderThreads)
+        order[atomicAdd(&bins[scratch[t]], 1)] = t;
+}
+
+cudaError_t longitude_order_launch(ls200_vectors *table) {
+    longitude_order_kernel<<<1, kOrderThreads, 0, table->ctx->stream>>>(
+        table->data, table->count, table->window, table->order);
+    return cudaGetLastError();
+}
+
 // window = the entries of `order` inside [t0, t0 + n), in order: one block,
 // each thread counting and then copying a contiguous run of `order` at the
 // offset given by a block scan of the counts.
-constexpr int kOrderThreads = 1024;
 
 __global__ void __launch_bounds__(kOrderThreads) order_window_kernel(
     const int *__restrict__ order, int count, int t0, int n, int *__restrict__ window) {

@@ -9,10 +9,11 @@
 // A Moon-ME vector table resident on the device (ls200_vectors_create).
 struct ls200_vectors {
     ls200_context *ctx = nullptr;
+    // One allocation: data, order, window.
     float *data = nullptr;  // device [count, 3]
     int count = 0;
-    // device [count]: time indices sorted by the vector's longitude
-    // atan2(y, x).  For a polar site the body's local azimuth follows its
+    // device [count]: time indices in the order of the vector's longitude
+    // atan2(y, x), to a bin of 0.044 degrees in a long table.  For a polar site the body's local azimuth follows its
     // longitude, so in this order consecutive steps read neighbouring
     // horizon bins.
     int *order = nullptr;
@@ -49,6 +50,9 @@ struct LightingBatch {
     const int *order;
 };
 
+// Fills table->order from table->data on the context's stream (window is its
+// scratch).
+cudaError_t longitude_order_launch(ls200_vectors *table);
 // With `table` (the vector table of the launch), fraction / byte / margin
 // launches visit their time steps in the table's longitude order.
 void lighting_launch(ls200_context *ctx, LightingBatch &batch, int tiles, int signal,

@@ -1,9 +1,7 @@
 // C-ABI entry points of the lighting products.
 #include "lighting.cuh"
 
-#include <algorithm>
 #include <cmath>
-#include <numeric>
 #include <vector>
 
 namespace ls200 {
@@ -27,8 +25,6 @@ void release_lighting_state(ls200_context *ctx) {
     if (!ctx->lighting) return;
     for (ls200_vectors *v : ctx->lighting->vectors) {
         tracked_free(v->data);
-        tracked_free(v->order);
-        tracked_free(v->window);
         delete v;
     }
     delete ctx->lighting;
@@ -64,38 +60,24 @@ ls200_status ls200_vectors_create(ls200_context *ctx, const float *vectors, int 
         LS_REQUIRE(count > 0, "at least one vector is required");
         std::lock_guard<std::mutex> hold(ctx->lock);
         activate(ctx);
-        // Time indices by longitude (ties by index); non-finite keys sort as 0.
-        std::vector<double> key(count);
-        for (int t = 0; t < count; ++t) {
-            const double k = std::atan2(static_cast<double>(vectors[3 * t + 1]),
-                                        static_cast<double>(vectors[3 * t]));
-            key[t] = std::isfinite(k) ? k : 0.0;
-        }
-        std::vector<int> order(count);
-        std::iota(order.begin(), order.end(), 0);
-        std::stable_sort(order.begin(), order.end(),
-                         [&](int a, int b) { return key[a] < key[b]; });
         auto v = new ls200_vectors();
         v->ctx = ctx;
         v->count = count;
         auto release = [&] {
             if (v->data) tracked_free(v->data);
-            if (v->order) tracked_free(v->order);
-            if (v->window) tracked_free(v->window);
             delete v;
         };
-        cudaError_t e = tracked_malloc(&v->data, sizeof(float) * 3 * size_t(count));
-        if (e == cudaSuccess) e = tracked_malloc(&v->order, sizeof(int) * size_t(count));
-        if (e == cudaSuccess) e = tracked_malloc(&v->window, sizeof(int) * size_t(count));
+        cudaError_t e = tracked_malloc(&v->data, (3 * sizeof(float) + 2 * sizeof(int)) *
+                                                     size_t(count));
         if (e != cudaSuccess) {
             release();
             throw Error(LS200_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
         }
+        v->order = reinterpret_cast<int *>(v->data + 3 * size_t(count));
+        v->window = v->order + count;
         e = cudaMemcpyAsync(v->data, vectors, sizeof(float) * 3 * size_t(count),
                             cudaMemcpyHostToDevice, ctx->stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(v->order, order.data(), sizeof(int) * size_t(count),
-                                cudaMemcpyHostToDevice, ctx->stream);
+        if (e == cudaSuccess) e = longitude_order_launch(v);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) {
             release();
@@ -114,8 +96,6 @@ ls200_status ls200_vectors_destroy(ls200_vectors *vectors) {
         cudaStreamSynchronize(vectors->ctx->stream);
         state_of(vectors->ctx).vectors.erase(vectors);
         tracked_free(vectors->data);
-        tracked_free(vectors->order);
-        tracked_free(vectors->window);
         delete vectors;
     });
 }
