@@ -20,9 +20,12 @@
 // eight sites 430 -> 390 ms).
 //
 // Launch configuration (autotuned, never changing results): how the 32 lanes
-// of a job map onto rays (L adjacent pixels x 32/L adjacent azimuths, L a
-// power of two up to 32), and the resident blocks per SM (8 at 64 registers,
-// 6 at 80; the relative march takes 7 for 8).
+// of a job map onto rays (L neighbouring pixels x 32/L adjacent azimuths, L a
+// power of two up to 32; 1x1, 2x1, 2x2, 4x2, 4x4 or 8x4 pixels), and the
+// resident blocks per SM (8 at 64 registers, 6 at 80; the relative march takes
+// 7 for 8).  The default of 2x2 pixels marches eight sites in 384.8 ms (ladder;
+// 2x1: 388, 4x1: 400, 4x2: 403) and two in 200.7 ms (exact; 2x1: 208.9, 4x1:
+// 201.3, 4x2: 199.8); the relative ladder's is 2x1 (two sites 74.2 ms, 2x2 75.3).
 #include "march_core.cuh"
 
 #include <map>
@@ -33,6 +36,7 @@ namespace ls200 {
 
 constexpr int kMaxSiteDems = 8;
 constexpr int kTileSide = 128;
+constexpr int kDefaultLanes = 4;  // BatchConfig's
 constexpr int kTilePixels = kTileSide * kTileSide;
 
 // Host-built description of one DEM; the level table is derived on the
@@ -144,10 +148,14 @@ __global__ void __launch_bounds__(128, kMinBlocks)
         const long long local = job - t * P.jobs_per_tile;
         const int azimuth_group = static_cast<int>(local / P.pixel_groups);
         const int pixel_group = static_cast<int>(local - azimuth_group * P.pixel_groups);
-        const int pixel = pixel_group * lanes + lane % lanes;
+        // Pixels in rectangles twice as wide as high, or square.
+        const int log_lanes = 31 - __clz(lanes), log_wide = (log_lanes + 1) >> 1;
+        const int across = kTileSide >> log_wide, sub = lane % lanes;
+        const int row = (pixel_group / across << (log_lanes - log_wide)) + (sub >> log_wide);
+        const int column = (pixel_group % across << log_wide) + (sub & ((1 << log_wide) - 1));
+        const int pixel = row * kTileSide + column;
         const int azimuth = azimuth_group * azimuths_per_job + lane / lanes;
         const BatchTile &tile = P.tiles[t];
-        const int row = pixel / kTileSide, column = pixel % kTileSide;
         const size_t ray = static_cast<size_t>(pixel) * P.azimuth_count + azimuth;
         float *out = tile.out + ray;
         const BatchDem &primary = P.dems[tile.dems[0]];
@@ -382,7 +390,9 @@ void march_sites_run(ls200_context *ctx, const ls200_site_tile *tiles, int tile_
         P.center_count = center_count;
         P.subpatch = subpatch_size;
         P.degrees = degrees ? 1 : 0;
-        P.lanes_per_azimuth = ctx->batch_lanes_per_azimuth;
+        P.lanes_per_azimuth = ctx->batch_lanes_per_azimuth ? ctx->batch_lanes_per_azimuth
+                              : traversal == (kLadderClimb | kRelative) ? 2
+                                                                        : kDefaultLanes;
         const int azimuths_per_job = 32 / P.lanes_per_azimuth;
         P.pixel_groups = kTilePixels / P.lanes_per_azimuth;
         P.jobs_per_tile = P.pixel_groups * ((azimuth_count + azimuths_per_job - 1) /
@@ -445,7 +455,8 @@ extern "C" ls200_status ls200_get_batch_config(ls200_context *ctx, int *lanes_pe
     return guard([&] {
         LS_REQUIRE(ctx && lanes_per_azimuth && min_blocks, "NULL argument");
         std::lock_guard<std::mutex> hold(ctx->lock);
-        *lanes_per_azimuth = ctx->batch_lanes_per_azimuth;
+        *lanes_per_azimuth = ctx->batch_lanes_per_azimuth ? ctx->batch_lanes_per_azimuth
+                                                          : kDefaultLanes;
         *min_blocks = ctx->batch_min_blocks;
     });
 }

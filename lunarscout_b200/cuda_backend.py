@@ -57,11 +57,11 @@ class SiteTile:
 @dataclass(frozen=True, slots=True)
 class BatchConfig:
     """Launch configuration of the persistent multi-site march:
-    ``lanes_per_azimuth`` adjacent pixels of one azimuth per 32-ray warp job
+    ``lanes_per_azimuth`` neighbouring pixels of one azimuth per 32-ray warp job
     (a power of two up to 32; the job spans 32/lanes azimuths) and ``min_blocks``
     resident 128-thread blocks per SM (8 at 64 registers or 6 at 80)."""
 
-    lanes_per_azimuth: int = 2
+    lanes_per_azimuth: int = 4
     min_blocks: int = 8
 
 
