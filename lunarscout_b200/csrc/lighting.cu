@@ -1088,7 +1088,10 @@ void mission_duration_launch(ls200_context *ctx, LightingBatch &B, int tiles,
 // The bits are taken a word at a time: the warp splits a word where the month
 // changes (the months are the same for every pixel), and within a part only
 // the ends of low-Sun runs are visited.  One step at a time was a chain of 25
-// instructions for each sample of a pixel.
+// instructions for each sample of a pixel; the scratch, a chain of memory
+// latencies at each run's end, is touched only where a run or the bits cross
+// into another month (kernel, two tiles, 17,545 hours: 420 us,
+// 485 with every run's end in memory).
 struct HavenParams {
     const uint32_t *low, *outage;  // [tiles, words, 16384]
     const int *month;              // [T] band of each time step, -1 for none
@@ -1125,18 +1128,31 @@ __global__ void __launch_bounds__(128) haven_kernel(const __grid_constant__ Have
     int lo = P.bands, hi = -1;       // bands the current run touched lie in [lo, hi]
     int cached = -1;                 // band whose flags sit in `bits`
     unsigned bits = 0u;
+    int top = 0;                     // longest credit of that band not yet in `longest`
+    bool spread = false;             // a stored band's flag 4 is set
     auto store = [&]() {
-        if (cached >= 0 && bits) flags[cached * plane] |= static_cast<uint8_t>(bits);
+        if (cached >= 0) {
+            if (bits) flags[cached * plane] |= static_cast<uint8_t>(bits);
+            if (top) longest[cached * plane] = max(longest[cached * plane], top);
+            spread = spread || (bits & 4u);
+        }
         bits = 0u;
+        top = 0;
     };
     auto credit = [&]() {
-        store();
-        for (int b = lo; b <= hi; ++b) {
-            const unsigned f = flags[b * plane];
-            if (f & 4u) {
-                longest[b * plane] = max(longest[b * plane], run);
-                flags[b * plane] = static_cast<uint8_t>(f & ~4u);
+        if (!spread) {  // a run inside one month: all of it in registers
+            top = max(top, run);
+            bits &= ~4u;
+        } else {
+            store();
+            for (int b = lo; b <= hi; ++b) {
+                const unsigned f = flags[b * plane];
+                if (f & 4u) {
+                    longest[b * plane] = max(longest[b * plane], run);
+                    flags[b * plane] = static_cast<uint8_t>(f & ~4u);
+                }
             }
+            spread = false;
         }
         lo = P.bands;
         hi = -1;
