@@ -25,9 +25,11 @@
 // resident blocks per SM (8 at 64 registers, 6 at 80; the relative march takes
 // 7 for 8).  The default of 2x2 pixels marches eight sites in 384.8 ms (ladder;
 // 2x1: 388, 4x1: 400, 4x2: 403) and two in 200.7 ms (exact; 2x1: 208.9, 4x1:
-// 201.3, 4x2: 199.8); the relative ladder's is 2x1 (two sites 74.2 ms, 2x2 75.3).
+// 201.3, 4x2: 199.8); the relative ladder's and that of full steps is 2x1 (two
+// sites, relative ladder: 74.2 ms, 2x2 75.3).
 #include "march_core.cuh"
 
+#include <algorithm>
 #include <map>
 #include <type_traits>
 #include <vector>
@@ -104,6 +106,14 @@ struct WarpLevels {
     __device__ __forceinline__ int4 cells(int l) const { return t.cells[l]; }
 };
 
+// The ladder with the full step throughout: march_dem_ladder tries each step
+// twice where the cell of the footprint's level is not culled, and on a large
+// fine DEM that is every third step.  Two tiles of a 5 m site, ladder_step
+// against full steps: 126 ms / 152 at 2048^2 pixels, 168 / 194 at 4096^2, but
+// 581 / 474 at 6144^2 and 606 / 515 at 8192^2.
+constexpr int kFullSteps = 4;
+constexpr int kSettledSide = 4096;  // largest DEM side for ladder_step (pixels)
+
 struct SitesBlock {
     RayStore::Block rays;
     WarpDem dems[4];
@@ -137,8 +147,8 @@ __global__ void __launch_bounds__(128, kMinBlocks)
     const int lanes = P.lanes_per_azimuth;
     const int azimuths_per_job = 32 / lanes;
     unsigned visits = 0, samples = 0, steps = 0;
-    __shared__ typename std::conditional<(kLadder & kRelative) == 0, SitesBlock, char>::type
-        store;
+    constexpr bool full_steps = (kLadder & (kRelative | kFullSteps)) != 0;
+    __shared__ typename std::conditional<!full_steps, SitesBlock, char>::type store;
     for (;;) {
         unsigned long long taken = 0;
         if (lane == 0) taken = atomicAdd(P.next_job, 1ull);
@@ -192,10 +202,11 @@ __global__ void __launch_bounds__(128, kMinBlocks)
                     primary_height, ratio);
             }
             if constexpr (kArgmax) tracker.current_pass = d;
-            if constexpr ((kLadder & kRelative) != 0) {
-                current = march_dem_tracked<kCount, kLadder>(GlobalLevels{&dem.table}, view, g, d,
-                                                             observer_z, current, visits, samples,
-                                                             steps, tracker);
+            if constexpr (full_steps) {
+                if (marches)
+                    current = march_dem_tracked<kCount, kLadder & ~kFullSteps>(
+                        GlobalLevels{&dem.table}, view, g, d, observer_z, current, visits, samples,
+                        steps, tracker);
             } else {
                 // The warp's own copy of the DEM's level table.
                 WarpDem &here = store.dems[threadIdx.x >> 5];
@@ -254,6 +265,9 @@ static void dispatch(ls200_context *ctx, const SitesParams &P, int traversal) {
     switch (traversal) {
         case kReference: launch_sites<kCount, kReference, kMinBlocks>(ctx, P); break;
         case kLadderClimb: launch_sites<kCount, kLadderClimb, kMinBlocks>(ctx, P); break;
+        case kLadderClimb | kFullSteps:
+            launch_sites<kCount, kLadderClimb | kFullSteps, kMinBlocks>(ctx, P);
+            break;
         case kRelative:
             // 64 registers spill too much here: 349.6 ms at 7 blocks for two
             // sites of 2048^2 over 3072^2, 353.4 at 8.
@@ -268,6 +282,8 @@ static void dispatch(ls200_context *ctx, const SitesParams &P, int traversal) {
 // one tile: 50 ms, 51 at 8).
 static void dispatch_argmax(ls200_context *ctx, const SitesParams &P, int traversal) {
     if (traversal == kReference) launch_sites<false, kReference, 7, true>(ctx, P);
+    else if (traversal & kFullSteps)
+        launch_sites<false, kLadderClimb | kFullSteps, 8, true>(ctx, P);
     else launch_sites<false, kLadderClimb, 7, true>(ctx, P);
 }
 
@@ -294,6 +310,7 @@ void march_sites_run(ls200_context *ctx, const ls200_site_tile *tiles, int tile_
         std::map<const ls200_dem *, int> index;
         std::vector<ls200_dem *> unique;
         size_t segment_floats = 0;
+        int largest = 0;
         for (int t = 0; t < tile_count; ++t) {
             const ls200_site_tile &tile = tiles[t];
             LS_REQUIRE(tile.dems && tile.dem_count > 0 && tile.dem_count <= kMaxSiteDems,
@@ -303,6 +320,7 @@ void march_sites_run(ls200_context *ctx, const ls200_site_tile *tiles, int tile_
                 LS_REQUIRE(dem != nullptr, "NULL DEM");
                 LS_REQUIRE(dem->ctx == ctx, "DEM belongs to another context");
                 LS_REQUIRE(dem->width >= 2 && dem->height >= 2, "DEMs must be at least 2x2 pixels");
+                largest = std::max({largest, dem->width, dem->height});
                 if (!index.count(dem)) {
                     index[dem] = static_cast<int>(unique.size());
                     unique.push_back(dem);
@@ -390,9 +408,10 @@ void march_sites_run(ls200_context *ctx, const ls200_site_tile *tiles, int tile_
         P.center_count = center_count;
         P.subpatch = subpatch_size;
         P.degrees = degrees ? 1 : 0;
+        if (traversal == kLadderClimb && largest > kSettledSide) traversal |= kFullSteps;
         P.lanes_per_azimuth = ctx->batch_lanes_per_azimuth ? ctx->batch_lanes_per_azimuth
-                              : traversal == (kLadderClimb | kRelative) ? 2
-                                                                        : kDefaultLanes;
+                              : traversal > kRelative ? 2
+                                                      : kDefaultLanes;
         const int azimuths_per_job = 32 / P.lanes_per_azimuth;
         P.pixel_groups = kTilePixels / P.lanes_per_azimuth;
         P.jobs_per_tile = P.pixel_groups * ((azimuth_count + azimuths_per_job - 1) /

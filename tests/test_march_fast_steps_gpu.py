@@ -136,3 +136,40 @@ def test_batched_settled_steps_keep_every_slope_and_decision(name, traversal, cu
     assert (visits, samples) == tuple(counts)
     for dem in device:
         dem.close()
+
+
+@pytest.mark.parametrize("height,width", [(4096, 300), (4097, 300), (300, 4097)])
+def test_ladder_on_both_sides_of_the_size_limit(height, width, cuda_session):
+    """DEMs with a side above 4096 pixels take full steps: the same slopes and
+    counters as the oracle's ladder."""
+    import torch
+
+    from lunarscout_b200.contract import PyramidArrays, map_parameters, projection_parameters
+    from lunarscout_b200.cuda_backend import SiteTile
+
+    dem = _dem(height, width, 5.0)
+    column, row, azimuths, distance = min(128, width - 140), 1024 % (height - 130), 8, 30_000.0
+    device = cuda_session.upload_dem_grid(dem)
+    tile = SiteTile((device,), column, row, distance, 2.0)
+    out = torch.empty(128 * 128 * azimuths, device="cuda")
+    torch.cuda.synchronize()
+    mips, levels = oracle.build_pyramid(dem.elevation_m)
+    pyramid = PyramidArrays(dem.elevation_m, mips, levels, map_parameters(dem),
+                            projection_parameters(dem))
+    segments = cuda_session.generate_segments(
+        [device], tile_column=column, tile_row=row, azimuth_count=azimuths,
+        maximum_distance_m=distance, observer_elevation_m=2.0)
+    expected, counts = oracle.march_all_passes(
+        segments, [pyramid], tile_column=column, tile_row=row, observer_elevation_m=2.0,
+        mask=oracle.ladder_mask(0, 1))
+    for counting in (False, True):
+        cuda_session.set_counting(counting)
+        try:
+            cuda_session.march_sites([tile], device_out=out.data_ptr(), azimuth_count=azimuths,
+                                     traversal="ladder")
+            counters = cuda_session.last_counters() if counting else None
+        finally:
+            cuda_session.set_counting(False)
+        np.testing.assert_array_equal(out.cpu().numpy().reshape(expected.shape), expected)
+    assert counters[:2] == tuple(counts)
+    device.close()
