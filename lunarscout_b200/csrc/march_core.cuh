@@ -19,8 +19,9 @@
 // equals the IEEE reciprocal on every input it receives (see rcp_approx).
 // The x and y arithmetic of a step (path position and tangent, planar
 // offset, cell-exit slab) is issued as f32x2 pairs, whose lanes round as the
-// scalar intrinsics do.  No shift amount is ever taken from stored state:
-// an amount out of range is undefined even on a path that is never taken.
+// scalar intrinsics do.  No shift amount comes from stored state unclamped:
+// an amount out of range is undefined even on a path that is never taken
+// (slow_step clamps the level that it loads).
 // With the same segment inputs the results are bit-identical to the CPU
 // oracle's FP32 restatement under its production mask.
 //
@@ -1400,7 +1401,9 @@ __device__ __forceinline__ void slow_step(FarCell &far, const RayStore &store, c
     const float z = store.get(RayStore::kObserver);
     const float limit = store.get(RayStore::kLimit);
     const float before = store.get(RayStore::kCurrent);
-    const int level = __float_as_int(store.get(RayStore::kLevel));
+    // Clamped: march_step shifts by it and indexes the level table with it.
+    const int level = min(max(__float_as_int(store.get(RayStore::kLevel)), 0),
+                          dem.level_count - 1);
     MarchState st{s, before, level, store.get(RayStore::kSideUp),
                   store.get(RayStore::kSideHere)};
     bool alive = true;
