@@ -1387,6 +1387,14 @@ __device__ __forceinline__ float march_near(const Table &table, const DemView &d
     return s;
 }
 
+// The last path position of a ray that RayStore holds.  Finite (or NaN): a ray
+// that has ended stands at +inf, which must lie past every end, also that of a
+// caller's segment without one.
+__device__ __forceinline__ float ray_end(const RaySegment &g) {
+    constexpr float kLargest = 0x1.fffffep127f;
+    return g.s_end > kLargest ? kLargest : g.s_end;
+}
+
 // The step of a lane that far_step left over: level0_step or the reference's
 // full step, and what they change for the next fast steps.
 template <bool kCount, bool kAhead, class Table, class Tracker>
@@ -1460,7 +1468,7 @@ __device__ __forceinline__ float march_dem_far(const Table &table, const DemView
     store.set(RayStore::kSideUp, first.side_up);
     store.set(RayStore::kSideHere, first.side_here);
     store.set(RayStore::kLevel, __int_as_float(first.level_hint));
-    store.set(RayStore::kEnd, g.s_end);
+    store.set(RayStore::kEnd, ray_end(g));
     store.set(RayStore::kChord, g.s_start_chord);
     store.set(RayStore::kObserver, observer_z);
     store.set(RayStore::kLimit, range.tame ? range.end : INFINITY);  // +inf: not tame
@@ -1647,7 +1655,7 @@ __device__ __forceinline__ float march_dem_ladder(const Table &table, const DemV
                ladder_sine(dem.radius + observer_z, current));
     store.save(1, g.s_start_chord * 1000.0f, 0.004363323129985824f / dem.resolution, current,
                0.0f);
-    store.set(RayStore::kEnd, g.s_end);
+    store.set(RayStore::kEnd, ray_end(g));
     store.set(RayStore::kChord, g.s_start_chord);
     store.set(RayStore::kLimit, tame ? 0.0f : INFINITY);  // +inf: not tame
     for (;;) {
