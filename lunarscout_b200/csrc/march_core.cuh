@@ -812,7 +812,8 @@ __device__ __forceinline__ void far_ahead(FarCell &far, float2 tangent) {
 }
 
 // The s range in which steps may settle.  The segment must keep the
-// approximations' error bounds (finite, of ordinary size, the chord
+// approximations' error bounds (finite, of ordinary size, starting at or
+// after the observer: march_near bounds the tangent from there; the chord
 // polynomial's higher terms within a fifth of its linear one, the path
 // bounded by its coefficients), the DEM must be small enough for exact float
 // cell edges, and the path must stay inside the DEM by more than its
@@ -837,9 +838,9 @@ __device__ __forceinline__ bool far_tame(const DemView &dem, const RaySegment &g
                                          float observer_z) {
     const float reach = path_reach(g);
     const float planar = reach * dem.resolution * 1.0001f;
-    return g.s_end - g.s_start >= 1e-3f && reach < 4e6f && fabsf(g.start.x) < 4e6f &&
-           fabsf(g.start.y) < 4e6f && g.s_start_chord >= 0.0f && g.s_start_chord < 1e6f &&
-           g.c1 >= 0.1f && g.c1 <= 10.0f &&
+    return g.s_start >= 0.0f && g.s_end - g.s_start >= 1e-3f && reach < 4e6f &&
+           fabsf(g.start.x) < 4e6f && fabsf(g.start.y) < 4e6f && g.s_start_chord >= 0.0f &&
+           g.s_start_chord < 1e6f && g.c1 >= 0.1f && g.c1 <= 10.0f &&
            planar * (fabsf(g.c2) + planar * fabsf(g.c3)) <= 0.2f * g.c1 &&
            dem.width <= (1 << 22) && dem.height <= (1 << 22) && fabsf(observer_z) < 1e6f &&
            dem.radius > 1e5f && dem.radius < 1e9f;

@@ -57,3 +57,22 @@ def test_device_segments_without_an_end(cuda_session):
     finally:
         device.close()
     np.testing.assert_array_equal(out.cpu().numpy(), expected)
+
+
+def test_a_path_that_starts_far_behind_its_first_sample(cuda_session):
+    """s_start = -3 km: from the first sample on (s = 1 m) the path's offset is
+    past 3 km, where a curved path's tangent has little to do with its start."""
+    _, pyramid, segments = _case(5.0)
+    k1 = segments[..., [4, 8]].copy()  # pixels per km at the sample
+    segments[..., [0, 1]] -= k1 * np.float32(3.0 - 9.0 / 6.6)
+    segments[..., [2, 3]] = segments[..., [0, 1]]
+    segments[..., 4:12] = 0.0
+    segments[..., [4, 8]] = k1
+    segments[..., [5, 9]] = -k1 / np.float32(6.6)
+    segments[..., 12] = -3.0
+    segments[..., 16:18] = 0.0
+    expected = _expected(segments, pyramid)
+    got, _ = cuda_session.subpatch_hierarchical_all_passes(
+        segments, [pyramid], tile_height=16, observer_elevation_m=2.0, **TILE)
+    assert np.isfinite(expected).mean() > 0.9
+    np.testing.assert_array_equal(got, expected)
