@@ -20,18 +20,33 @@ StagedCopies::~StagedCopies() {
     if (slots_) cudaFreeHost(slots_);
 }
 
-void StagedCopies::open() {
-    if (!slots_)
-        LS_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&slots_), kThreads * kSlot,
-                              cudaHostAllocPortable));
-    for (cudaStream_t &s : streams_)
-        if (!s) LS_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    if (!ready_) LS_CUDA(cudaEventCreateWithFlags(&ready_, cudaEventDisableTiming));
+int StagedCopies::open() {
+    if (!slots_ && cudaHostAlloc(reinterpret_cast<void **>(&slots_), kThreads * kSlot,
+                                 cudaHostAllocPortable) != cudaSuccess)
+        slots_ = nullptr;
+    if (!ready_ && cudaEventCreateWithFlags(&ready_, cudaEventDisableTiming) != cudaSuccess)
+        ready_ = nullptr;
+    int streams = 0;
+    for (; slots_ && ready_ && streams < kThreads; ++streams) {
+        cudaStream_t &s = streams_[streams];
+        if (!s && cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) {
+            s = nullptr;
+            break;
+        }
+    }
+    if (streams < kThreads) cudaGetLastError();  // a refusal here fails no copy
+    return streams;
 }
 
 void StagedCopies::run(int device, bool to_host, char *host, char *gpu, size_t bytes,
                        cudaStream_t after) {
-    open();
+    const int streams = open();
+    if (streams == 0) {
+        LS_CUDA(cudaMemcpyAsync(to_host ? host : gpu, to_host ? gpu : host, bytes,
+                                to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, after));
+        LS_CUDA(cudaStreamSynchronize(after));
+        return;
+    }
     LS_CUDA(cudaEventRecord(ready_, after));
     std::atomic<size_t> next{0};
     std::atomic<int> failure{cudaSuccess};
@@ -56,7 +71,7 @@ void StagedCopies::run(int device, bool to_host, char *host, char *gpu, size_t b
     const size_t pieces = (bytes + kSlot - 1) / kSlot;
     const size_t cores = std::max(1u, std::thread::hardware_concurrency());
     const int workers =
-        static_cast<int>(std::max<size_t>(1, std::min({size_t(kThreads), pieces, cores})));
+        static_cast<int>(std::max<size_t>(1, std::min({size_t(streams), pieces, cores})));
     std::vector<std::thread> threads;
     threads.reserve(workers);
     for (int w = 1; w < workers; ++w) {

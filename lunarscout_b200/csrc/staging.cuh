@@ -9,7 +9,9 @@
 namespace ls200 {
 
 // Owned by a context (its calls are serialised); slots and streams are made
-// on first use and released with it.
+// on first use and released with it.  A host that will not page-lock the slots
+// (10 MB; a small locked-memory limit) or a driver without a stream to spare
+// gets the driver's own copy, one that has some streams as many threads.
 class StagedCopies {
 public:
     ~StagedCopies();
@@ -21,7 +23,7 @@ public:
 private:
     static constexpr int kThreads = 10;  // at most; never more than the host has cores
     static constexpr size_t kSlot = size_t(1) << 20;
-    void open();
+    int open();  // the streams there are; 0: no slots, no event or no stream
     void run(int device, bool to_host, char *host, char *gpu, size_t bytes, cudaStream_t after);
     char *slots_ = nullptr;  // kThreads x kSlot, page-locked
     cudaStream_t streams_[kThreads] = {};
