@@ -184,8 +184,10 @@ ls200_status ls200_march_sites(ls200_context *ctx, const ls200_site_tile *tiles,
  * not depend on it): `lanes_per_azimuth` = how many neighbouring pixels of one
  * azimuth a 32-ray warp job holds (a power of two from 1 to 32; the job then
  * spans 32 / lanes_per_azimuth azimuths), `min_blocks` = resident 128-thread blocks per SM, 8 (64
- * registers) or 6 (80 registers).  Chosen by the autotuner; defaults 4, 8 (the
- * relative ladder takes 2 lanes until a configuration is set). */
+ * registers) or 6 (80 registers).  Chosen by the autotuner.  Until one is set
+ * the lanes are 0, each traversal's own (4; 2 for the relative ladder and for
+ * the ladder over DEMs of more than 4096 pixels a side), and the blocks 8;
+ * what ls200_get_batch_config gives can be set again. */
 ls200_status ls200_set_batch_config(ls200_context *ctx, int lanes_per_azimuth, int min_blocks);
 ls200_status ls200_get_batch_config(ls200_context *ctx, int *lanes_per_azimuth, int *min_blocks);
 

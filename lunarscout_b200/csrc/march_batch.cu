@@ -38,7 +38,7 @@ namespace ls200 {
 
 constexpr int kMaxSiteDems = 8;
 constexpr int kTileSide = 128;
-constexpr int kDefaultLanes = 4;  // BatchConfig's
+constexpr int kDefaultLanes = 4;  // of the traversals with settled steps; 2 of the others
 constexpr int kTilePixels = kTileSide * kTileSide;
 
 // Host-built description of one DEM; the level table is derived on the
@@ -459,9 +459,10 @@ extern "C" ls200_status ls200_set_batch_config(ls200_context *ctx, int lanes_per
                                                int min_blocks) {
     return guard([&] {
         LS_REQUIRE(ctx, "NULL argument");
-        LS_REQUIRE(lanes_per_azimuth >= 1 && lanes_per_azimuth <= 32 &&
+        LS_REQUIRE(lanes_per_azimuth >= 0 && lanes_per_azimuth <= 32 &&
                        (lanes_per_azimuth & (lanes_per_azimuth - 1)) == 0,
-                   "lanes_per_azimuth must be a power of two from 1 to 32");
+                   "lanes_per_azimuth must be a power of two from 1 to 32, or 0 for each "
+                   "traversal's own");
         LS_REQUIRE(min_blocks == 6 || min_blocks == 8, "min_blocks must be 6 or 8");
         std::lock_guard<std::mutex> hold(ctx->lock);
         ctx->batch_lanes_per_azimuth = lanes_per_azimuth;
@@ -474,8 +475,7 @@ extern "C" ls200_status ls200_get_batch_config(ls200_context *ctx, int *lanes_pe
     return guard([&] {
         LS_REQUIRE(ctx && lanes_per_azimuth && min_blocks, "NULL argument");
         std::lock_guard<std::mutex> hold(ctx->lock);
-        *lanes_per_azimuth = ctx->batch_lanes_per_azimuth ? ctx->batch_lanes_per_azimuth
-                                                          : kDefaultLanes;
+        *lanes_per_azimuth = ctx->batch_lanes_per_azimuth;
         *min_blocks = ctx->batch_min_blocks;
     });
 }

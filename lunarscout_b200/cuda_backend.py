@@ -58,7 +58,8 @@ class SiteTile:
 class BatchConfig:
     """Launch configuration of the persistent multi-site march:
     ``lanes_per_azimuth`` neighbouring pixels of one azimuth per 32-ray warp job
-    (a power of two up to 32; the job spans 32/lanes azimuths) and ``min_blocks``
+    (a power of two up to 32; the job spans 32/lanes azimuths; 0, what a session
+    has until one is set, leaves it to the traversal) and ``min_blocks``
     resident 128-thread blocks per SM (8 at 64 registers or 6 at 80)."""
 
     lanes_per_azimuth: int = 4
