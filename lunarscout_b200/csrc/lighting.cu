@@ -186,6 +186,11 @@ static int ordered_chunk(int chunk, int time_count) {
 // Margins: the approximate direction is within 4e-7 rad (2.3e-5 deg) of the
 // exact one in both its own and the reference's rounding, for bodies at least
 // 50 planet radii away (checked per chunk; nearer ones take the exact path).
+// Near the vertical that error, relative to the whole vector, is not small
+// against its horizontal part, and the azimuth is lost: a step settles only
+// where the horizontal part exceeds a thousandth of the chunk's longest vector
+// (below 89.94 deg: 0.1 bin).  A chunk with a vector whose square is beyond a
+// float's range settles nothing.
 // Taking the angle for its sine is 0.11 bin off at the window's end (8 deg).
 // An entry therefore covers one bin more than a sample reads and is chosen half
 // a bin low.  The elevations keep 1.2e-3 deg (kClear), of which the exact
@@ -229,6 +234,7 @@ struct WindowAxes {
     float2 x, y, z, t;     // (across, along) per vector component, translation
     float ux, uy, uz, ut;  // up
     float position;        // of the middle, in entries
+    float least;           // horizontal length that a settled step needs
 };
 
 // A step's vector as the packed arithmetic wants it: (x, x, y, y) and
@@ -242,7 +248,8 @@ struct StagedVector {
 };
 
 // Sine of the angle from the window's middle and tangent of the elevation;
-// returns whether the body is on the middle's side.
+// returns whether the body is on the middle's side and far enough from the
+// vertical.
 __device__ __forceinline__ bool approximate_direction(const WindowAxes &w, const StagedVector &v,
                                                       float &sine, float &tangent) {
     float2 h = __ffma2_rn(make_float2(v.xy.x, v.xy.y), w.x, w.t);
@@ -253,7 +260,7 @@ __device__ __forceinline__ bool approximate_direction(const WindowAxes &w, const
     const float inverse = rsqrtf(__fmaf_rn(h.x, h.x, h.y * h.y));
     sine = h.x * inverse;
     tangent = up * inverse;
-    return h.y > 0.0f;
+    return h.y > w.least;
 }
 
 // Shared memory of a staged launch's block.
@@ -262,6 +269,7 @@ struct StagedBlock {
     float4 vectors[2 * kMaxChunk];
     uint16_t queue[4][64];                 // undecided samples: step << 5 | lane
     int far;                               // every vector is 50 radii away
+    unsigned longest;                      // bits of the largest squared length
     __device__ __forceinline__ StagedVector vector(int k) const {
         return StagedVector{vectors[2 * k], vectors[2 * k + 1]};
     }
@@ -290,6 +298,7 @@ __device__ __forceinline__ int stage_entries(StagedBlock &S, const Frame32 &f,
     w.y = make_float2(f.v[3] * cos_a - f.v[4] * sin_a, f.v[3] * sin_a + f.v[4] * cos_a);
     w.z = make_float2(f.v[6] * cos_a - f.v[7] * sin_a, f.v[6] * sin_a + f.v[7] * cos_a);
     w.t = make_float2(f.v[9] * cos_a - f.v[10] * sin_a, f.v[9] * sin_a + f.v[10] * cos_a);
+    w.least = 1e-3f * sqrtf(__uint_as_float(S.longest));
     w.ux = f.v[2], w.uy = f.v[5], w.uz = f.v[8], w.ut = f.v[11];
     w.position = azimuth_deg * 4.0f - (kSpan == 5 ? 1.58f : 0.0f);
     float low = w.position, high = w.position;
@@ -371,10 +380,11 @@ __device__ __forceinline__ int stage_entries(StagedBlock &S, const Frame32 &f,
 template <class Op>
 __device__ __forceinline__ void stage_vectors(StagedBlock &S, const LightingBatch &B, int k0,
                                               int steps, const Op &op) {
-    if (threadIdx.x == 0) S.far = 1;
+    if (threadIdx.x == 0) S.far = 1, S.longest = 0u;
     __syncthreads();
     const float scale = 1.0f / (50.0f * fabsf(static_cast<float>(B.tiles[blockIdx.z].proj[0])) +
                                 1.0f);
+    unsigned longest = 0u;  // positive floats order as their bits; NaN is above +inf
     for (int k = threadIdx.x; k < steps; k += blockDim.x) {
         const int t = __ldg(B.order + k0 + k);
         const float *v = B.vectors + 3 * static_cast<size_t>(t);
@@ -385,7 +395,11 @@ __device__ __forceinline__ void stage_vectors(StagedBlock &S, const LightingBatc
             make_float4(z, z, __uint_as_float(words.x), __uint_as_float(words.y));
         const float sx = x * scale, sy = y * scale, sz = z * scale;
         if (!(sx * sx + sy * sy + sz * sz >= 1.0f)) S.far = 0;
+        const float squared = x * x + y * y + z * z;
+        longest = max(longest, __float_as_uint(squared < 1e38f ? squared : INFINITY));
     }
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    if ((threadIdx.x & 31) == 0) atomicMax(&S.longest, longest);
     __syncthreads();
 }
 
