@@ -127,32 +127,45 @@ __device__ __forceinline__ Frame32 load_frame(const float *frames, size_t pixel)
 constexpr int kWindowBins = 32;
 constexpr int kWindowStride = kWindowBins + 1;
 
-// Stage the bins that the margins at positions [k0, k1) of the launch's order
-// read (two from each step's first bin) into `window`; returns the number
-// staged (0: none) and sets `first`, the window's first bin.  In longitude
-// order the body's azimuth moves monotonically across a chunk, so the bins
-// between those of its first and last steps, plus the span and a margin of 2
-// on each side, cover it; a step outside them reads its row directly.
+template <int kSpan>
+__device__ __forceinline__ BinPosition signal_position(float azimuth_deg) {
+    return kSpan == 5 ? sun_position(azimuth_deg) : margin_position(azimuth_deg);
+}
+
+// The sun fraction (kSpan 5) or the margin (kSpan 2) of a pixel.
+template <int kSpan, class Bins>
+__device__ __forceinline__ float signal_bins(const Bins &bin, float fraction, float elevation) {
+    return kSpan == 5 ? sun_fraction_bins(bin, fraction, elevation)
+                      : horizon_margin_bins(bin, fraction, elevation);
+}
+
+// Stage the bins that positions [k0, k1) of the launch's order read (kSpan
+// bins from each step's first bin: 2 for the margin, 5 for the fraction)
+// into `window`; returns the number staged (0: none) and sets `first`, the
+// window's first bin.  In longitude order the body's azimuth moves
+// monotonically across a chunk, so the bins between those of its first and
+// last steps, plus the span and a margin of 2 on each side, cover it; a step
+// outside them reads its row directly.
+template <int kSpan>
 __device__ __forceinline__ int stage_window(const LightingBatch &B, const Frame32 &f,
                                             const float *horizon, int k0, int k1, float *window,
                                             int &first) {
-    if (!B.order || k1 <= k0) return 0;
     float azimuth_deg, elevation;
     const float *v = B.vectors + 3 * static_cast<size_t>(__ldg(B.order + k0));
     body_direction(f, __ldg(v), __ldg(v + 1), __ldg(v + 2), azimuth_deg, elevation);
-    const int a = margin_position(azimuth_deg).left;
+    const int a = signal_position<kSpan>(azimuth_deg).left;
     v = B.vectors + 3 * static_cast<size_t>(__ldg(B.order + k1 - 1));
     body_direction(f, __ldg(v), __ldg(v + 1), __ldg(v + 2), azimuth_deg, elevation);
-    const int b = margin_position(azimuth_deg).left;
+    const int b = signal_position<kSpan>(azimuth_deg).left;
     int arc = b - a;
     if (arc < 0) arc += kAzimuths;
     int start = arc <= kAzimuths / 2 ? a : b;
     if (arc > kAzimuths / 2) arc = kAzimuths - arc;
     start -= 2;
     if (start < 0) start += kAzimuths;
-    if (arc + 6 > kWindowBins) return 0;
+    const int width = arc + kSpan + 4;
+    if (width > kWindowBins) return 0;
     first = start;
-    const int width = arc + 6;
     for (int i = 0; i < width; ++i) {
         int bin = first + i;
         if (bin >= kAzimuths) bin -= kAzimuths;
@@ -161,10 +174,125 @@ __device__ __forceinline__ int stage_window(const LightingBatch &B, const Frame3
     return width;
 }
 
-// Chunk length of an ordered launch: a chunk of c steps sweeps about
-// c * 1440 / T bins; keep that to 20 so its bins fit the staged window.
+// Evaluates positions [k0, k1) of the launch's order for one pixel and calls
+// put(time index, signal); `windowed`: with the bins staged (ordered launches).
+// The loops are unrolled as measured: a margin's (3 steps without a window, 4
+// with one) keep several row reads in flight, 16 patches of 125 and 1460 steps of
+// a year 429 and 3055 us against 710 and 4175 with the loops left to the
+// compiler; fractions take 2 and 1, bytes 2 and 2 (1 % better than others, and 4
+// is 7 % worse).
+template <int kSpan, int kDirectUnroll, int kWindowUnroll, class Put>
+__device__ __forceinline__ void exact_samples(const LightingBatch &B, const Frame32 &f,
+                                              const float *horizon, int k0, int k1,
+                                              bool windowed, float *window, const Put &put) {
+    auto direction = [&](int k, float &azimuth_deg, float &elevation) {
+        const int t = B.order ? __ldg(B.order + k) : B.time_start + k;
+        const float *v = B.vectors + 3 * static_cast<size_t>(t);
+        body_direction(f, __ldg(v), __ldg(v + 1), __ldg(v + 2), azimuth_deg, elevation);
+        return t;
+    };
+    int first = 0, width = 0;
+    if (windowed && k0 < k1) width = stage_window<kSpan>(B, f, horizon, k0, k1, window, first);
+    // One loop for the warp: a lane without a window goes along with the others'.
+    if (!__any_sync(__activemask(), width > 0)) {
+#pragma unroll kDirectUnroll
+        for (int k = k0; k < k1; ++k) {
+            float azimuth_deg, elevation;
+            const int t = direction(k, azimuth_deg, elevation);
+            const BinPosition p = signal_position<kSpan>(azimuth_deg);
+            put(t, signal_bins<kSpan>(GlobalBins{horizon, p.left}, p.fraction, elevation));
+        }
+        return;
+    }
+#pragma unroll kWindowUnroll
+    for (int k = k0; k < k1; ++k) {
+        float azimuth_deg, elevation;
+        const int t = direction(k, azimuth_deg, elevation);
+        const BinPosition p = signal_position<kSpan>(azimuth_deg);
+        int offset = p.left - first;
+        if (offset < 0) offset += kAzimuths;
+        float signal;
+        if (offset + kSpan <= width)
+            signal = signal_bins<kSpan>(SharedBins{window, offset}, p.fraction, elevation);
+        else
+            signal = signal_bins<kSpan>(GlobalBins{horizon, p.left}, p.fraction, elevation);
+        put(t, signal);
+    }
+}
+
+// The steps of a block of an exact launch.  Short chunks hide the latency of
+// the row reads; a window costs two directions and its bins, and pays from some
+// 16 steps on that read the same bins.  So B.group chunks of B.chunk steps form
+// a group: where its first and last vectors lie close together in longitude, the
+// first of its blocks takes all of it with a window and the others end; where
+// not, each takes its own chunk without one.  Close: as many bins as a window
+// holds, and no more than the window saves (2 a step for the fraction, which
+// reads 5; 0.75 for the margin, which reads 2).  Four patches, 355 steps of a
+// year and of a day: fractions 461 and 360 us (a window tried in every chunk of
+// 16: 469 and 358; chunks of 10 without windows: 433 and 487), margins 239 and
+// 198 us (366 and 200; a window tried in every chunk of 10: 280 and 205).
+struct ExactSteps {
+    int first, last;
+    bool windowed;
+};
+
+template <int kSpan>
+__device__ __forceinline__ ExactSteps exact_steps(const LightingBatch &B) {
+    const int y = blockIdx.y;
+    if (B.group == 0) return ExactSteps{y * B.chunk, min((y + 1) * B.chunk, B.time_count), false};
+    // The first parts of all groups come first: they have the most to do.
+    const int groups = gridDim.y / B.group, part = y / groups;
+    const int g0 = (y - part * groups) * B.group * B.chunk;
+    const int g1 = min(g0 + B.group * B.chunk, B.time_count);
+    const float *a = B.vectors + 3 * static_cast<size_t>(__ldg(B.order + g0));
+    const float *b = B.vectors + 3 * static_cast<size_t>(__ldg(B.order + g1 - 1));
+    const float ax = __ldg(a), ay = __ldg(a + 1), bx = __ldg(b), by = __ldg(b + 1);
+    const float bins = kSpan == 5 ? fminf(24.0f, 2.0f * (g1 - g0))
+                                  : fminf(24.0f, 0.75f * (g1 - g0));
+    // (A NaN, or vectors a quarter turn apart, is not close.)  0.25 deg a bin.
+    if (fabsf(ax * by - ay * bx) <= 4.36e-3f * bins * (ax * bx + ay * by))
+        return ExactSteps{g0, part ? g0 : g1, true};
+    return ExactSteps{min(g0 + part * B.chunk, g1), min(g0 + (part + 1) * B.chunk, g1), false};
+}
+
+// Chunk length of an ordered launch with windows: a chunk of c steps sweeps
+// about c * 1440 / T bins; keep that to 20 so its bins fit the window.
 static int ordered_chunk(int chunk, int time_count) {
     return std::min(chunk, std::max(16, (kWindowBins - 12) * time_count / kAzimuths));
+}
+
+// Enough (pixel-block x chunk x tile) blocks for ~8 waves of 128-thread
+// blocks on every SM, chunks of at least `least` time steps.
+static int lighting_chunk(ls200_context *ctx, int tiles, int time_count, int least) {
+    const int blocks_per_chunk = (kPatch * kPatch / 128) * tiles;
+    const int want = ctx->props.multiProcessorCount * 16 * 8;
+    int chunks = std::max(1, want / std::max(1, blocks_per_chunk));
+    chunks = std::min(chunks, std::max(1, time_count / least));
+    return (time_count + chunks - 1) / chunks;
+}
+
+// Sets the chunks of an exact launch and returns how many there are.  At least 4
+// steps a chunk: a short table's launch is bound by the latency of its row reads
+// (125 steps of one patch took 56 us in chunks of 16, 47 in chunks of 5: 32-byte
+// sectors of 2 M rows).  Ordered launches take about 24 blocks per SM where that
+// leaves shorter chunks than windows want, and groups of the latter's length;
+// but none where the groups' first blocks alone would leave the chip idle (one
+// patch, 125 steps of an hour: 76 us without, 79 with).
+static int exact_chunks(ls200_context *ctx, LightingBatch &B, int tiles) {
+    B.chunk = lighting_chunk(ctx, tiles, B.time_count, 4);
+    B.group = 0;
+    if (!B.order) return (B.time_count + B.chunk - 1) / B.chunk;
+    const int blocks = (kPatch * kPatch / 128) * tiles, sms = ctx->props.multiProcessorCount;
+    const int windowed = ordered_chunk(lighting_chunk(ctx, tiles, B.time_count, 16), B.time_count);
+    const int chunks = std::max(1, sms * 24 / blocks);
+    const int small = std::max(4, (B.time_count + chunks - 1) / chunks);
+    const int parts = std::max(1, (windowed + small - 1) / small);
+    B.chunk = (windowed + parts - 1) / parts;
+    if (static_cast<long long>(B.time_count / windowed) * blocks < sms * 8)
+        return (B.time_count + B.chunk - 1) / B.chunk;
+    B.group = parts;
+    const int steps = parts * B.chunk;
+    return (B.time_count + steps - 1) / steps * parts;
 }
 
 // ---------------------------------------------------------------------------
@@ -405,8 +533,8 @@ __device__ __forceinline__ void stage_vectors(StagedBlock &S, const LightingBatc
 
 // Visits every sample of the block: op.settled(words, high) where the entries
 // decide the thread's own pixel, op.outside(words) where that lies outside the
-// valid rectangle (!valid), and op.exact(pixel offset, frame, horizon, vector,
-// words) otherwise, for a pixel of the thread's warp.
+// valid rectangle (!valid), and op.put(pixel offset, signal, words) otherwise,
+// for a pixel of the thread's warp.
 template <int kSpan, class Op>
 __device__ __forceinline__ void staged_samples(StagedBlock &S, const LightingBatch &B, bool valid,
                                                float shift, float clearance, Op &op) {
@@ -468,8 +596,16 @@ __device__ __forceinline__ void staged_samples(StagedBlock &S, const LightingBat
                 const int entry = queue[lane];
                 const int offset = (entry & 31) - lane;
                 const StagedVector v = S.vector(entry >> 5);
-                op.exact(offset, load_frame(B.frames, pixel + offset),
-                         B.horizons + (pixel + offset) * kAzimuths, v.vector(), v.words());
+                const float3 body = v.vector();
+                float azimuth_deg, elevation;
+                body_direction(load_frame(B.frames, pixel + offset), body.x, body.y, body.z,
+                               azimuth_deg, elevation);
+                const BinPosition p = signal_position<kSpan>(azimuth_deg);
+                op.put(offset,
+                       signal_bins<kSpan>(
+                           GlobalBins{B.horizons + (pixel + offset) * kAzimuths, p.left},
+                           p.fraction, elevation),
+                       v.words());
             }
             __syncwarp();
             if (lane + n < pending) queue[lane] = queue[lane + n];
@@ -479,12 +615,13 @@ __device__ __forceinline__ void staged_samples(StagedBlock &S, const LightingBat
     }
 }
 
-// Longest chunk of a staged launch: about 20 bins of azimuth, so that its
-// entries fit.  Launches below kStagedSteps steps spend more on staging than
+// Sets the chunks of a staged launch, about 20 bins of azimuth, so that their
+// entries fit, and returns how many there are.  Launches below kStagedSteps steps spend more on staging than
 // they save: one patch takes 212 us against 342 at 720 steps, 236 either way
 // at 360.
-static int staged_chunk(int time_count) {
-    return std::max(4, std::min(kMaxChunk, static_cast<int>(20ll * time_count / kAzimuths)));
+static int staged_chunks(LightingBatch &B) {
+    B.chunk = std::max(4, std::min(kMaxChunk, static_cast<int>(20ll * B.time_count / kAzimuths)));
+    return (B.time_count + B.chunk - 1) / B.chunk;
 }
 constexpr int kStagedSteps = 720;
 // (Rows are staged in 16-byte quads, and a word plane's 32-bit offset bounds
@@ -495,7 +632,8 @@ static bool staged_launch(const LightingBatch &B) {
 }
 
 // Fractions (float32 or bytes) into the launch's time-major output; the words
-// of a step are its plane's 64-bit offset.
+// of a step are its plane's 64-bit offset.  step() is the same by time index
+// for the exact kernels.
 template <class T>
 struct StoreSample {
     T *out;  // the thread's pixel in the first plane
@@ -516,11 +654,11 @@ struct StoreSample {
         *place(w) = high ? static_cast<T>(sizeof(T) == 1 ? 255 : 1) : static_cast<T>(0);
     }
     __device__ __forceinline__ void outside(uint2 w) const { *place(w) = static_cast<T>(0); }
-    __device__ __forceinline__ void exact(int offset, const Frame32 &f, const float *horizon,
-                                          float3 v, uint2 w) const {
-        float azimuth_deg, elevation;
-        body_direction(f, v.x, v.y, v.z, azimuth_deg, elevation);
-        place(w)[offset] = value(sun_fraction(horizon, azimuth_deg, elevation));
+    __device__ __forceinline__ void put(int offset, float signal, uint2 w) const {
+        place(w)[offset] = value(signal);
+    }
+    __device__ __forceinline__ void step(int t, float signal) const {
+        out[static_cast<size_t>(t - time_start) * (kPatch * kPatch)] = value(signal);
     }
 };
 
@@ -546,61 +684,28 @@ __global__ void __launch_bounds__(128, kStagedBlocks)
     staged_samples<5>(S, B, valid, 0.0f, c_half_circle[7] + kClear, op);
 }
 
-// Margins, and fractions of launches that are not staged.  Margins stage each
-// chunk's bins (stage_window); a short or unordered launch of fractions reads
-// its rows directly.
-template <int kSignal>
+// Margins, and fractions of launches that are not staged: every sample exactly.
+template <int kSpan, class T>
 __global__ void __launch_bounds__(128) lighting_kernel(const __grid_constant__ LightingBatch B) {
+    __shared__ float windows[128 * kWindowStride];
     const int tile = blockIdx.z;
-    const int index = blockIdx.x * blockDim.x + threadIdx.x;
-    if (index >= kPatch * kPatch) return;
+    const int index = blockIdx.x * 128 + threadIdx.x;
     const TileGeo &g = B.tiles[tile];
-    const int sample = index % kPatch, line = index / kPatch;
-    // Chunk blockIdx.y covers positions [k0, k1) of the launch's order.
-    const int k0 = blockIdx.y * B.chunk;
-    const int k1 = min(k0 + B.chunk, B.time_count);
-    const size_t plane = static_cast<size_t>(kPatch) * kPatch;
-    const size_t tile_out = static_cast<size_t>(tile) * B.time_count * plane;
-    if (sample >= g.valid_width || line >= g.valid_height) {
-        for (int k = k0; k < k1; ++k) {
-            const int t = B.order ? __ldg(B.order + k) : B.time_start + k;
-            const size_t o = tile_out + static_cast<size_t>(t - B.time_start) * plane + index;
-            if (kSignal == kSignalBytes) static_cast<uint8_t *>(B.out)[o] = 0;
-            else static_cast<float *>(B.out)[o] = 0.0f;
-        }
+    const ExactSteps steps = exact_steps<kSpan>(B);
+    const StoreSample<T> op{static_cast<T *>(B.out) +
+                                static_cast<size_t>(tile) * B.time_count * (kPatch * kPatch) +
+                                index,
+                            B.time_start};
+    if (index % kPatch >= g.valid_width || index / kPatch >= g.valid_height) {
+        for (int k = steps.first; k < steps.last; ++k)
+            op.step(B.order ? __ldg(B.order + k) : B.time_start + k, 0.0f);
         return;
     }
-    const size_t pixel = static_cast<size_t>(tile) * plane + index;
-    const Frame32 f = load_frame(B.frames, pixel);
-    const float *horizon = B.horizons + pixel * kAzimuths;
-    constexpr bool kMargin = kSignal == kSignalMargin;
-    __shared__ float windows[kMargin ? 128 * kWindowStride : 1];
-    float *window = windows + (kMargin ? threadIdx.x * kWindowStride : 0);
-    int first = 0;
-    const int width = kMargin ? stage_window(B, f, horizon, k0, k1, window, first) : 0;
-    for (int k = k0; k < k1; ++k) {
-        const int t = B.order ? __ldg(B.order + k) : B.time_start + k;
-        const float *v = B.vectors + 3 * static_cast<size_t>(t);
-        float azimuth_deg, elevation;
-        body_direction(f, __ldg(v), __ldg(v + 1), __ldg(v + 2), azimuth_deg, elevation);
-        const size_t o = tile_out + static_cast<size_t>(t - B.time_start) * plane + index;
-        if (kMargin) {
-            const BinPosition p = margin_position(azimuth_deg);
-            int offset = p.left - first;
-            if (offset < 0) offset += kAzimuths;
-            static_cast<float *>(B.out)[o] =
-                offset + 2 <= width
-                    ? horizon_margin_bins(SharedBins{window, offset}, p.fraction, elevation)
-                    : horizon_margin_bins(GlobalBins{horizon, p.left}, p.fraction, elevation);
-        } else {
-            const float visible = sun_fraction(horizon, azimuth_deg, elevation);
-            if (kSignal == kSignalBytes)
-                static_cast<uint8_t *>(B.out)[o] =
-                    static_cast<uint8_t>(static_cast<int>(__fmul_rn(255.0f, visible)));
-            else
-                static_cast<float *>(B.out)[o] = visible;
-        }
-    }
+    const size_t pixel = static_cast<size_t>(tile) * kPatch * kPatch + index;
+    exact_samples<kSpan, kSpan == 2 ? 3 : 2, kSpan == 2 ? 4 : sizeof(T) == 1 ? 2 : 1>(
+        B, load_frame(B.frames, pixel), B.horizons + pixel * kAzimuths, steps.first, steps.last,
+        steps.windowed, windows + threadIdx.x * kWindowStride,
+        [&](int t, float signal) { op.step(t, signal); });
 }
 
 // PSR (psr_cuda.py:57-186): 255 unless a reduced vector's centre rises above
@@ -660,18 +765,6 @@ __global__ void sun_fraction_kernel(const float *horizons, const float *azimuth_
     if (i >= n) return;
     out[i] = sun_fraction(horizons + static_cast<size_t>(i) * kAzimuths, azimuth_deg[i],
                           elevation_deg[i]);
-}
-
-int lighting_chunk(ls200_context *ctx, int tiles, int time_count) {
-    // Enough (pixel-block x chunk x tile) blocks for ~8 waves of 128-thread
-    // blocks on every SM, chunks of at least 4 time steps (a short table's
-    // launch is bound by the latency of its row reads: 125 steps of one patch
-    // took 56 us in chunks of 16, 47 in chunks of 5: 32-byte sectors of 2 M rows).
-    const int blocks_per_chunk = (kPatch * kPatch / 128) * tiles;
-    const int want = ctx->props.multiProcessorCount * 16 * 8;
-    int chunks = std::max(1, want / std::max(1, blocks_per_chunk));
-    chunks = std::min(chunks, std::max(1, time_count / 4));
-    return (time_count + chunks - 1) / chunks;
 }
 
 // The time indices of a table in longitude order, to a bin of 0.044 degrees (a
@@ -785,22 +878,19 @@ void lighting_launch(ls200_context *ctx, LightingBatch &B, int tiles, int signal
         dim3 grid(kPatch * kPatch / kPsrWarps, 1, tiles);
         psr_kernel<<<grid, kPsrWarps * 32, 0, ctx->stream>>>(B);
     } else if (staged_launch(B) && signal != kSignalMargin) {
-        B.chunk = staged_chunk(B.time_count);
-        dim3 grid(kPatch * kPatch / 128, (B.time_count + B.chunk - 1) / B.chunk, tiles);
+        dim3 grid(kPatch * kPatch / 128, staged_chunks(B), tiles);
         if (signal == kSignalBytes)
             staged_fraction_kernel<uint8_t><<<grid, 128, 0, ctx->stream>>>(B);
         else
             staged_fraction_kernel<float><<<grid, 128, 0, ctx->stream>>>(B);
     } else {
-        B.chunk = lighting_chunk(ctx, tiles, B.time_count);
-        if (B.order) B.chunk = ordered_chunk(B.chunk, B.time_count);
-        dim3 grid(kPatch * kPatch / 128, (B.time_count + B.chunk - 1) / B.chunk, tiles);
+        dim3 grid(kPatch * kPatch / 128, exact_chunks(ctx, B, tiles), tiles);
         if (signal == kSignalFraction)
-            lighting_kernel<kSignalFraction><<<grid, 128, 0, ctx->stream>>>(B);
+            lighting_kernel<5, float><<<grid, 128, 0, ctx->stream>>>(B);
         else if (signal == kSignalBytes)
-            lighting_kernel<kSignalBytes><<<grid, 128, 0, ctx->stream>>>(B);
+            lighting_kernel<5, uint8_t><<<grid, 128, 0, ctx->stream>>>(B);
         else
-            lighting_kernel<kSignalMargin><<<grid, 128, 0, ctx->stream>>>(B);
+            lighting_kernel<2, float><<<grid, 128, 0, ctx->stream>>>(B);
     }
     LS_CUDA(cudaGetLastError());
 }
@@ -836,7 +926,7 @@ void directions_launch(ls200_context *ctx, LightingBatch &B, int tiles, float2 *
     dim3 grid_frames(kPatch * kPatch / 128, tiles);
     frames_kernel<<<grid_frames, 128, 0, ctx->stream>>>(B);
     LS_CUDA(cudaGetLastError());
-    B.chunk = lighting_chunk(ctx, tiles, B.time_count);
+    B.chunk = lighting_chunk(ctx, tiles, B.time_count, 4);
     dim3 grid(kPatch * kPatch / 128, (B.time_count + B.chunk - 1) / B.chunk, tiles);
     directions_kernel<<<grid, 128, 0, ctx->stream>>>(B, out);
     LS_CUDA(cudaGetLastError());
@@ -848,13 +938,6 @@ void directions_launch(ls200_context *ctx, LightingBatch &B, int tiles, float2 *
 // margin.  Each thread visits a chunk of the body's table in its longitude
 // order and sets the bits of its steps with atomicOr (other chunks own the
 // word's other steps).  Each signal runs in its own body's order.
-template <int kSpan>
-__device__ __forceinline__ float signal_value(const float *horizon, float azimuth_deg,
-                                              float elevation) {
-    return kSpan == 5 ? sun_fraction(horizon, azimuth_deg, elevation)
-                      : horizon_margin(horizon, azimuth_deg, elevation);
-}
-
 template <bool kAtLeast>
 __device__ __forceinline__ bool passes(float value, float threshold) {
     return kAtLeast ? value >= threshold : value < threshold;
@@ -873,12 +956,12 @@ struct SetBit {
         if (is_high ? high : low) atomicOr(bits + w.x, w.y);
     }
     __device__ __forceinline__ void outside(uint2) const {}
-    __device__ __forceinline__ void exact(int offset, const Frame32 &f, const float *horizon,
-                                          float3 v, uint2 w) const {
-        float azimuth_deg, elevation;
-        body_direction(f, v.x, v.y, v.z, azimuth_deg, elevation);
-        if (passes<kAtLeast>(signal_value<kSpan>(horizon, azimuth_deg, elevation), threshold))
-            atomicOr(bits + offset + w.x, w.y);
+    __device__ __forceinline__ void put(int offset, float signal, uint2 w) const {
+        if (passes<kAtLeast>(signal, threshold)) atomicOr(bits + offset + w.x, w.y);
+    }
+    __device__ __forceinline__ void step(int t, float signal) const {
+        if (passes<kAtLeast>(signal, threshold))
+            atomicOr(bits + static_cast<size_t>(t >> 5) * (kPatch * kPatch), 1u << (t & 31));
     }
 };
 
@@ -904,25 +987,19 @@ template <int kSpan, bool kAtLeast>
 __global__ void __launch_bounds__(128) signal_bits_kernel(const __grid_constant__ LightingBatch B,
                                                           float threshold, int words,
                                                           uint32_t *__restrict__ bits) {
-    const int tile = blockIdx.z;
-    const int index = blockIdx.x * blockDim.x + threadIdx.x;
-    const TileGeo &g = B.tiles[tile];
+    __shared__ float windows[128 * kWindowStride];
+    const int index = blockIdx.x * 128 + threadIdx.x;
+    const TileGeo &g = B.tiles[blockIdx.z];
     if (index % kPatch >= g.valid_width || index / kPatch >= g.valid_height) return;
-    const size_t plane = static_cast<size_t>(kPatch) * kPatch;
-    uint32_t *tile_bits = bits + static_cast<size_t>(tile) * words * plane + index;
-    const int k0 = blockIdx.y * B.chunk;
-    const int k1 = min(k0 + B.chunk, B.time_count);
-    const size_t pixel = static_cast<size_t>(tile) * plane + index;
-    const Frame32 f = load_frame(B.frames, pixel);
-    const float *horizon = B.horizons + pixel * kAzimuths;
-    for (int k = k0; k < k1; ++k) {
-        const int t = B.order ? __ldg(B.order + k) : k;
-        const float *v = B.vectors + 3 * static_cast<size_t>(t);
-        float azimuth_deg, elevation;
-        body_direction(f, __ldg(v), __ldg(v + 1), __ldg(v + 2), azimuth_deg, elevation);
-        if (passes<kAtLeast>(signal_value<kSpan>(horizon, azimuth_deg, elevation), threshold))
-            atomicOr(tile_bits + static_cast<size_t>(t >> 5) * plane, 1u << (t & 31));
-    }
+    const size_t pixel = static_cast<size_t>(blockIdx.z) * kPatch * kPatch + index;
+    const SetBit<kSpan, kAtLeast> op{
+        bits + static_cast<size_t>(blockIdx.z) * words * (kPatch * kPatch) + index, threshold,
+        false, false};
+    const ExactSteps steps = exact_steps<kSpan>(B);
+    exact_samples<kSpan, kSpan == 2 ? 3 : 1, kSpan == 2 ? 4 : 1>(
+        B, load_frame(B.frames, pixel), B.horizons + pixel * kAzimuths, steps.first, steps.last,
+        steps.windowed, windows + threadIdx.x * kWindowStride,
+        [&](int t, float signal) { op.step(t, signal); });
 }
 
 // Zero `bits` ([tiles, words, 16384] words) and set the threshold bits of
@@ -938,8 +1015,8 @@ static void signal_bits_launch(ls200_context *ctx, LightingBatch B, int tiles,
     B.vectors = vectors;
     B.order = order;
     const bool staged = staged_launch(B);
-    B.chunk = staged ? staged_chunk(B.time_count) : lighting_chunk(ctx, tiles, B.time_count);
-    dim3 grid(kPatch * kPatch / 128, (B.time_count + B.chunk - 1) / B.chunk, tiles);
+    dim3 grid(kPatch * kPatch / 128,
+              staged ? staged_chunks(B) : exact_chunks(ctx, B, tiles), tiles);
     if (staged)
         staged_bits_kernel<kSpan, kAtLeast>
             <<<grid, 128, 0, ctx->stream>>>(B, threshold, words, bits);
@@ -1292,12 +1369,11 @@ struct CountVisible {
     __device__ __forceinline__ uint2 words(int) const { return make_uint2(0u, 0u); }
     __device__ __forceinline__ void settled(uint2, bool high) { count += high ? 1u : 0u; }
     __device__ __forceinline__ void outside(uint2) const {}
-    __device__ __forceinline__ void exact(int offset, const Frame32 &f, const float *horizon,
-                                          float3 v, uint2) const {
-        float azimuth_deg, elevation;
-        body_direction(f, v.x, v.y, v.z, azimuth_deg, elevation);
-        if (horizon_margin(horizon, azimuth_deg, elevation) >= threshold)
-            atomicAdd(counts + offset, 1u);
+    __device__ __forceinline__ void put(int offset, float signal, uint2) const {
+        if (signal >= threshold) atomicAdd(counts + offset, 1u);
+    }
+    __device__ __forceinline__ void step(int, float signal) {
+        count += signal >= threshold ? 1u : 0u;
     }
 };
 
@@ -1318,24 +1394,17 @@ __global__ void __launch_bounds__(128, kStagedBlocks)
 __global__ void __launch_bounds__(128) visibility_kernel(const __grid_constant__ LightingBatch B,
                                                          float threshold,
                                                          unsigned *__restrict__ counts) {
-    const int tile = blockIdx.z;
-    const int index = blockIdx.x * blockDim.x + threadIdx.x;
-    const TileGeo &g = B.tiles[tile];
+    __shared__ float windows[128 * kWindowStride];
+    const int index = blockIdx.x * 128 + threadIdx.x;
+    const TileGeo &g = B.tiles[blockIdx.z];
     if (index % kPatch >= g.valid_width || index / kPatch >= g.valid_height) return;
-    const int k0 = blockIdx.y * B.chunk;
-    const int k1 = min(k0 + B.chunk, B.time_count);
-    const size_t pixel = static_cast<size_t>(tile) * kPatch * kPatch + index;
-    const Frame32 f = load_frame(B.frames, pixel);
-    const float *horizon = B.horizons + pixel * kAzimuths;
-    unsigned count = 0;
-    for (int k = k0; k < k1; ++k) {
-        const int t = B.order ? __ldg(B.order + k) : k;
-        const float *v = B.vectors + 3 * static_cast<size_t>(t);
-        float azimuth_deg, elevation;
-        body_direction(f, __ldg(v), __ldg(v + 1), __ldg(v + 2), azimuth_deg, elevation);
-        count += horizon_margin(horizon, azimuth_deg, elevation) >= threshold ? 1u : 0u;
-    }
-    if (count) atomicAdd(counts + pixel, count);
+    const size_t pixel = static_cast<size_t>(blockIdx.z) * kPatch * kPatch + index;
+    CountVisible op{counts + pixel, threshold, 0u};
+    const ExactSteps steps = exact_steps<2>(B);
+    exact_samples<2, 3, 4>(B, load_frame(B.frames, pixel), B.horizons + pixel * kAzimuths, steps.first,
+                     steps.last, steps.windowed, windows + threadIdx.x * kWindowStride,
+                     [&](int t, float signal) { op.step(t, signal); });
+    if (op.count) atomicAdd(op.counts, op.count);
 }
 
 __global__ void visibility_finalize(const unsigned *__restrict__ counts, int n, int time_count,
@@ -1359,8 +1428,8 @@ void visibility_launch(ls200_context *ctx, LightingBatch &B, int tiles, float th
     frames_kernel<<<grid_frames, 128, 0, ctx->stream>>>(B);
     LS_CUDA(cudaGetLastError());
     const bool staged = staged_launch(B);
-    B.chunk = staged ? staged_chunk(B.time_count) : lighting_chunk(ctx, tiles, B.time_count);
-    dim3 grid(kPatch * kPatch / 128, (B.time_count + B.chunk - 1) / B.chunk, tiles);
+    dim3 grid(kPatch * kPatch / 128,
+              staged ? staged_chunks(B) : exact_chunks(ctx, B, tiles), tiles);
     if (staged)
         staged_visibility_kernel<<<grid, 128, 0, ctx->stream>>>(B, threshold, counts);
     else

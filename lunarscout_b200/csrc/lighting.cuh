@@ -44,7 +44,8 @@ struct LightingBatch {
     const float *vectors;    // [T, 3] float32 Moon-ME metres
     float *frames;           // [tiles, 16384, 12]
     void *out;               // [tiles, time_count, 16384] (PSR: [tiles, 16384])
-    int time_start, time_count, chunk;
+    int time_start, time_count;
+    int chunk, group;        // steps per block, chunks per group (exact_steps)
     // [time_count] the launch's time indices in processing order, or NULL
     // for time order; outputs stay in time order either way.
     const int *order;
@@ -168,12 +169,6 @@ __device__ __forceinline__ float horizon_margin_bins(const Bins &bin, float frac
                                                      float elevation) {
     const float hl = bin(0), hr = bin(1);
     return __fsub_rn(elevation, __fadd_rn(hl, __fmul_rn(fraction, __fsub_rn(hr, hl))));
-}
-
-__device__ __forceinline__ float horizon_margin(const float *horizon, float azimuth_deg,
-                                                float elevation) {
-    const BinPosition p = margin_position(azimuth_deg);
-    return horizon_margin_bins(GlobalBins{horizon, p.left}, p.fraction, elevation);
 }
 
 // Visible fraction of the solar disk: 16 vertical slices of a 0.27-deg disk
