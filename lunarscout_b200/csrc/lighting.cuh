@@ -18,6 +18,7 @@ struct ls200_vectors {
     // horizon bins.
     int *order = nullptr;
     int *window = nullptr;  // device [count]: one launch's sub-range of `order`
+    float shortest = 0.0f;  // length of the shortest vector (m; 0 with a NaN)
 };
 
 namespace ls200 {
@@ -49,6 +50,7 @@ struct LightingBatch {
     // [time_count] the launch's time indices in processing order, or NULL
     // for time order; outputs stay in time order either way.
     const int *order;
+    float shortest;  // the ordered table's (ls200_vectors)
 };
 
 // Fills table->order from table->data on the context's stream (window is its
@@ -72,34 +74,32 @@ void directions_launch(ls200_context *ctx, LightingBatch &batch, int tiles, floa
 // per start interval into out [tiles, I, 16384] (hours, or days).  hours:
 // device [T] sample durations; prefix: device [T + 1] exact prefix sums or
 // NULL; windows: device [I] (first, end) sample indices of each start
-// window; order / earth_order: the Sun's / Earth's table in longitude order
-// (NULL: time order), the order in which each signal is evaluated.
+// window.  Each signal is evaluated in its own table's longitude order.
 void mission_duration_launch(ls200_context *ctx, LightingBatch &batch, int tiles,
-                             const float *earth, float sun_threshold, float earth_threshold,
-                             uint32_t *bits, const double *hours, const double *prefix,
-                             const int2 *windows, int interval_count, bool days, float *out,
-                             const int *order, const int *earth_order);
+                             const ls200_vectors *sun, const ls200_vectors *earth,
+                             float sun_threshold, float earth_threshold, uint32_t *bits,
+                             const double *hours, const double *prefix, const int2 *windows,
+                             int interval_count, bool days, float *out);
 
 // The safe-haven product fused with the lighting: low-Sun and Earth-outage
 // bits ([2, tiles, ceil(T/32), 16384] words in `bits`), then per pixel and
 // month band the longest low-Sun run that overlapped an outage in that band,
 // in hours, into out [tiles, bands, 16384] (NaN where the band is ill-posed).
 // month: device [T] band index per time step (-1 for none); longest and
-// flags: device scratch [tiles, bands, 16384]; order / earth_order: the
-// Sun's / Earth's table in longitude order (NULL: time order), the order in
-// which each body's bits are evaluated.
-void safe_haven_launch(ls200_context *ctx, LightingBatch &batch, int tiles, const float *earth,
+// flags: device scratch [tiles, bands, 16384].
+void safe_haven_launch(ls200_context *ctx, LightingBatch &batch, int tiles,
+                       const ls200_vectors *sun, const ls200_vectors *earth,
                        float sunlight_threshold, float earth_threshold, uint32_t *bits,
-                       const int *month, int bands, float hours, int *longest,
-                       uint8_t *flags, float *out, const int *order, const int *earth_order);
+                       const int *month, int bands, float hours, int *longest, uint8_t *flags,
+                       float *out);
 
 // Earth-visibility fraction: per pixel the share of the batch's time steps
 // whose Earth margin is >= threshold (degrees), into out [tiles, 16384] (NaN
 // outside the valid rectangle).  counts: device scratch [tiles, 16384];
-// valid: device [tiles] (valid width, valid height); order: the table's
-// longitude order of the time steps (NULL: time order).
-void visibility_launch(ls200_context *ctx, LightingBatch &batch, int tiles, float threshold,
-                       unsigned *counts, int2 *valid, float *out, const int *order);
+// valid: device [tiles] (valid width, valid height).
+void visibility_launch(ls200_context *ctx, LightingBatch &batch, int tiles,
+                       const ls200_vectors *earth, float threshold, unsigned *counts,
+                       int2 *valid, float *out);
 
 #ifdef LS200_LIGHTING_KERNELS
 // Slice half-heights and their normaliser (set by ensure_lighting_constants).

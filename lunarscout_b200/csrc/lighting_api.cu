@@ -1,6 +1,7 @@
 // C-ABI entry points of the lighting products.
 #include "lighting.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -35,6 +36,18 @@ static void check_valid(int valid_width, int valid_height) {
     LS_REQUIRE(valid_width >= 1 && valid_width <= kPatch && valid_height >= 1 &&
                    valid_height <= kPatch,
                "valid patch dimensions must be between 1 and 128");
+}
+
+// The length of the shortest vector, or 0 with a NaN among them.
+static float shortest_length(const float *vectors, int count) {
+    float least = INFINITY;
+    for (int t = 0; t < count; ++t) {
+        const float *v = vectors + 3 * static_cast<size_t>(t);
+        const float squared = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
+        if (std::isnan(squared)) return 0.0f;
+        least = std::min(least, squared);
+    }
+    return std::sqrt(least);
 }
 
 static LightingBatch single_batch(LightingState &st, const ls200_vectors *v) {
@@ -78,6 +91,7 @@ ls200_status ls200_vectors_create(ls200_context *ctx, const float *vectors, int 
         e = cudaMemcpyAsync(v->data, vectors, sizeof(float) * 3 * size_t(count),
                             cudaMemcpyHostToDevice, ctx->stream);
         if (e == cudaSuccess) e = longitude_order_launch(v);
+        v->shortest = shortest_length(vectors, count);  // while the device sorts
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) {
             release();
@@ -290,11 +304,10 @@ ls200_status ls200_mission_duration_device(
         B.frames = st.duration_frames.as<float>();
         B.time_start = 0;
         B.time_count = count;
-        mission_duration_launch(ctx, B, tile_count, earth ? earth->data : nullptr,
-                                sun_threshold, earth_threshold, st.duration_bits.as<uint32_t>(),
-                                d_hours, integral ? d_prefix : nullptr, d_windows,
-                                interval_count, output_days != 0, out, sun->order,
-                                earth ? earth->order : nullptr);
+        mission_duration_launch(ctx, B, tile_count, sun, earth, sun_threshold, earth_threshold,
+                                st.duration_bits.as<uint32_t>(), d_hours,
+                                integral ? d_prefix : nullptr, d_windows, interval_count,
+                                output_days != 0, out);
         // The host tables above must outlive their copies.
         LS_CUDA(cudaStreamSynchronize(ctx->stream));
     });
@@ -356,11 +369,10 @@ ls200_status ls200_safe_haven_device(
         B.frames = st.duration_frames.as<float>();
         B.time_start = 0;
         B.time_count = count;
-        safe_haven_launch(ctx, B, tile_count, earth->data, sunlight_threshold,
+        safe_haven_launch(ctx, B, tile_count, sun, earth, sunlight_threshold,
                           earth_threshold_deg, st.haven_bits.as<uint32_t>(),
                           st.haven_months.as<int32_t>(), band_count, time_step_hours,
-                          st.haven_longest.as<int32_t>(), st.haven_flags.as<uint8_t>(), out,
-                          sun->order, earth->order);
+                          st.haven_longest.as<int32_t>(), st.haven_flags.as<uint8_t>(), out);
         // The host month table must outlive its copy.
         LS_CUDA(cudaStreamSynchronize(ctx->stream));
     });
@@ -408,8 +420,8 @@ ls200_status ls200_earth_visibility_device(ls200_context *ctx, int tile_count,
         B.frames = st.duration_frames.as<float>();
         B.time_start = 0;
         B.time_count = earth->count;
-        visibility_launch(ctx, B, tile_count, threshold_deg, st.visibility.as<unsigned>(),
-                          d_valid, out, earth->order);
+        visibility_launch(ctx, B, tile_count, earth, threshold_deg,
+                          st.visibility.as<unsigned>(), d_valid, out);
         // The host valid table must outlive its copy.
         LS_CUDA(cudaStreamSynchronize(ctx->stream));
     });
