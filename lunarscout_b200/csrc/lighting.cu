@@ -710,52 +710,95 @@ __global__ void __launch_bounds__(128) lighting_kernel(const __grid_constant__ L
 }
 
 // PSR (psr_cuda.py:57-186): 255 unless a reduced vector's centre rises above
-// the interpolated horizon minus 0.545/2 deg.  One warp per pixel, a vector
-// per lane, until any lane is lit.  The lanes' vectors lie a 32nd of the table
-// apart, so each round looks in 32 directions and a lit pixel usually ends in
-// the first rounds; a shadowed one takes count / 32 rounds of the warp instead
-// of `count` of one thread, which held its whole launch (four patches, 2100
-// vectors: 1388 us with a thread per pixel).
+// the interpolated horizon minus 0.545/2 deg.
+__device__ __forceinline__ bool psr_lit(const Frame32 &f, const float *horizon, const float *v) {
+    float azimuth_deg, elevation;
+    body_direction(f, __ldg(v), __ldg(v + 1), __ldg(v + 2), azimuth_deg, elevation);
+    float position = __fmul_rn(azimuth_deg, 4.0f);
+    if (position >= static_cast<float>(kAzimuths)) position = 0.0f;
+    const int lower = static_cast<int>(position);
+    const float fraction = __fsub_rn(position, static_cast<float>(lower));
+    const int upper = lower + 1 >= kAzimuths ? 0 : lower + 1;
+    const float h1 = __ldg(horizon + lower), h2 = __ldg(horizon + upper);
+    const float h = __fadd_rn(h1, __fmul_rn(fraction, __fsub_rn(h2, h1)));
+    return __fsub_rn(elevation, h) > -0.2725f;
+}
+
+__device__ __forceinline__ bool psr_valid(const LightingBatch &B, int index) {
+    const TileGeo &g = B.tiles[blockIdx.z];
+    return index % kPatch < g.valid_width && index / kPatch < g.valid_height;
+}
+
+// One warp per pixel, a vector per lane, until any lane is lit.  The lanes'
+// vectors lie a 32nd of the table apart, so each round looks in 32 directions and
+// a lit pixel usually ends in the first rounds; a shadowed one takes count / 32
+// rounds of the warp instead of `count` of one thread, which held its whole
+// launch (four patches, 2100 vectors: 1388 us with a thread per pixel).
+// kLooked: psr_look_kernel has run, and only the pixels it left dark are open.
 constexpr int kPsrWarps = 8;
 
+template <bool kLooked>
 __global__ void __launch_bounds__(kPsrWarps * 32)
     psr_kernel(const __grid_constant__ LightingBatch B) {
-    const int tile = blockIdx.z;
     const int lane = threadIdx.x & 31;
     const int index = blockIdx.x * kPsrWarps + (threadIdx.x >> 5);
-    const TileGeo &g = B.tiles[tile];
-    const int sample = index % kPatch, line = index / kPatch;
-    uint8_t *out = static_cast<uint8_t *>(B.out) + static_cast<size_t>(tile) * kPatch * kPatch;
-    if (sample >= g.valid_width || line >= g.valid_height) {
-        if (lane == 0) out[index] = 0;
+    const size_t pixel = static_cast<size_t>(blockIdx.z) * kPatch * kPatch + index;
+    uint8_t *out = static_cast<uint8_t *>(B.out) + pixel;
+    if (kLooked ? *out == 0 : !psr_valid(B, index)) {
+        if (!kLooked && lane == 0) *out = 0;
         return;
     }
-    const size_t pixel = static_cast<size_t>(tile) * kPatch * kPatch + index;
     const Frame32 f = load_frame(B.frames, pixel);
     const float *horizon = B.horizons + pixel * kAzimuths;
     const int rounds = (B.time_count + 31) / 32;
-    bool lit = false;
     for (int r = 0; r < rounds; ++r) {
         const int t = lane * rounds + r;
-        if (t < B.time_count) {
-            const float *v = B.vectors + 3 * static_cast<size_t>(t);
-            float azimuth_deg, elevation;
-            body_direction(f, __ldg(v), __ldg(v + 1), __ldg(v + 2), azimuth_deg, elevation);
-            float position = __fmul_rn(azimuth_deg, 4.0f);
-            if (position >= static_cast<float>(kAzimuths)) position = 0.0f;
-            const int lower = static_cast<int>(position);
-            const float fraction = __fsub_rn(position, static_cast<float>(lower));
-            const int upper = lower + 1 >= kAzimuths ? 0 : lower + 1;
-            const float h1 = __ldg(horizon + lower), h2 = __ldg(horizon + upper);
-            const float h = __fadd_rn(h1, __fmul_rn(fraction, __fsub_rn(h2, h1)));
-            lit = __fsub_rn(elevation, h) > -0.2725f;
-        }
+        const bool lit = t < B.time_count &&
+                         psr_lit(f, horizon, B.vectors + 3 * static_cast<size_t>(t));
         if (__any_sync(0xffffffffu, lit)) {
-            if (lane == 0) out[index] = 0;
+            if (lane == 0) *out = 0;
             return;
         }
     }
-    if (lane == 0) out[index] = 255;
+    if (!kLooked && lane == 0) *out = 255;
+}
+
+// A look by one thread per pixel, at `looks` vectors spread over the table: all
+// of a short table, or a first one, which decides most lit pixels of a launch
+// whose warps would fill the chip several times.  Whole calls of four patches
+// (with a thread per pixel throughout; with warps only): 100 vectors, lit
+// 116 us (114; 129), dark 185 (228; 174); 8 vectors 129 (130; 140).
+constexpr int kPsrLookTiles = 3;   // patches of a launch from which on it looks first
+constexpr int kPsrShort = 16;      // table that it then looks at wholly
+constexpr int kPsrLooks = 2;
+
+__global__ void __launch_bounds__(128) psr_look_kernel(const __grid_constant__ LightingBatch B,
+                                                       int looks) {
+    const int index = blockIdx.x * 128 + threadIdx.x;
+    const size_t pixel = static_cast<size_t>(blockIdx.z) * kPatch * kPatch + index;
+    bool lit = !psr_valid(B, index);  // 0 outside the valid rectangle too
+    if (!lit) {
+        const Frame32 f = load_frame(B.frames, pixel);
+        for (int i = 0; i < looks && !lit; ++i) {
+            const int t = static_cast<int>(static_cast<long long>(B.time_count) * i / looks);
+            lit = psr_lit(f, B.horizons + pixel * kAzimuths,
+                          B.vectors + 3 * static_cast<size_t>(t));
+        }
+    }
+    static_cast<uint8_t *>(B.out)[pixel] = lit ? 0 : 255;
+}
+
+static void psr_launch(ls200_context *ctx, const LightingBatch &B, int tiles) {
+    const dim3 grid(kPatch * kPatch / kPsrWarps, 1, tiles);
+    if (tiles < kPsrLookTiles) {
+        psr_kernel<false><<<grid, kPsrWarps * 32, 0, ctx->stream>>>(B);
+        return;
+    }
+    const int looks = B.time_count <= kPsrShort ? B.time_count : kPsrLooks;
+    psr_look_kernel<<<dim3(kPatch * kPatch / 128, 1, tiles), 128, 0, ctx->stream>>>(B, looks);
+    if (looks == B.time_count) return;
+    LS_CUDA(cudaGetLastError());
+    psr_kernel<true><<<grid, kPsrWarps * 32, 0, ctx->stream>>>(B);
 }
 
 // Diagnostic: sun fraction for given (azimuth, elevation) per horizon row
@@ -877,8 +920,7 @@ void lighting_launch(ls200_context *ctx, LightingBatch &B, int tiles, int signal
     frames_kernel<<<grid_frames, 128, 0, ctx->stream>>>(B);
     LS_CUDA(cudaGetLastError());
     if (signal == kSignalPsr) {
-        dim3 grid(kPatch * kPatch / kPsrWarps, 1, tiles);
-        psr_kernel<<<grid, kPsrWarps * 32, 0, ctx->stream>>>(B);
+        psr_launch(ctx, B, tiles);
     } else if (signal != kSignalMargin && staged_launch(B, tiles)) {
         dim3 grid(kPatch * kPatch / 128, staged_chunks(B), tiles);
         if (signal == kSignalBytes)
