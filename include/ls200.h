@@ -406,8 +406,10 @@ ls200_status ls200_fp32_probe(ls200_context *ctx, int iterations, double *tflops
 /* Exhaustive check of the march's correctly rounded reciprocal (a hardware
  * approximation plus one Newton-Raphson correction) against the IEEE
  * round-to-nearest reciprocal on this device, over every 32-bit pattern with
- * |x| >= 2^-64, both signs: `mismatches` = results that differ in any bit
- * (must be 0), `checked` = results compared.  No reference counterpart. */
+ * |x| >= 2^-64, both signs, and of its division by 1000 against the IEEE one on
+ * the positive patterns from 2^-64 to 2^64: `mismatches` = results that differ
+ * in any bit (must be 0), `checked` = reciprocals compared.  No reference
+ * counterpart. */
 ls200_status ls200_check_arithmetic(ls200_context *ctx, int64_t *mismatches, int64_t *checked);
 
 /* Device memory held by this library's own allocations on `device` (DEMs,

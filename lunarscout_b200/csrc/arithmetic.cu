@@ -2,8 +2,10 @@
 // (reciprocal_pair in march_core.cuh: hardware approximation plus one
 // Newton-Raphson step) against the IEEE sequence __frcp_rn, bit for bit, on
 // every 32-bit pattern with |x| >= 2^-64 (the march uses it for |x| > 1e-8).
-// The march's bit parity with the reference rests on it; a GPU test and the
-// smoke check run it on the device the march runs on.
+// The same for its division by 1000 (over_1000: a faithful quotient corrected by
+// its residual) against __fdiv_rn, on every positive pattern from 2^-64 to 2^64.
+// The march's bit parity with the reference rests on them; a GPU test and the
+// smoke check run this on the device the march runs on.
 #include "march_core.cuh"
 
 namespace ls200 {
@@ -22,6 +24,8 @@ __global__ void arithmetic_check_kernel(unsigned long long *counts) {
         const float2 paired = reciprocal_pair(pair(x, -x));
         mismatches += __float_as_uint(paired.x) != __float_as_uint(__frcp_rn(x));
         mismatches += __float_as_uint(paired.y) != __float_as_uint(__frcp_rn(-x));
+        if (x < 0x1p64f)
+            mismatches += __float_as_uint(over_1000(x)) != __float_as_uint(__fdiv_rn(x, 1000.0f));
     }
     if (mismatches) atomicAdd(counts, mismatches);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(counts + 1, 2 * kCount);

@@ -923,8 +923,10 @@ __device__ __forceinline__ bool far_step(const FarCell &far, const RayStore &sto
 }
 
 // x / 1000 correctly rounded (for normal x and quotient): a faithful quotient
-// corrected by its exact residual (Markstein, as rcp_approx); equal to the
-// IEEE division for every significand.
+// corrected by its exact residual (Markstein, as rcp_approx).  Equal to the IEEE
+// division on every pattern from 2^-64 to 2^64 (ls200_check_arithmetic).  Its
+// operand is a path advance (m): 0 or at most a few kilometres, and a value too
+// small for the check loses to the floor step.
 __device__ __forceinline__ float over_1000(float x) {
     const float q = __fmul_rn(x, 0.001f);
     return __fmaf_rn(__fmaf_rn(-1000.0f, q, x), 0.001f, q);

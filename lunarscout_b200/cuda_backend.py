@@ -415,7 +415,9 @@ class CudaSession:
     def check_arithmetic(self) -> tuple[int, int]:
         """(mismatches, checked): results of the march's Newton reciprocal
         that differ in any bit from the IEEE reciprocal, over every pattern
-        with |x| >= 2^-64 and both signs; mismatches must be 0."""
+        with |x| >= 2^-64 and both signs (`checked` counts these), and of its
+        division by 1000 over the positive patterns from 2^-64 to 2^64;
+        mismatches must be 0."""
         mismatches, checked = ctypes.c_int64(), ctypes.c_int64()
         call("ls200_check_arithmetic", self._ctx, ctypes.byref(mismatches),
              ctypes.byref(checked))
