@@ -15,7 +15,8 @@ namespace ls200 {
 class StagedCopies {
 public:
     ~StagedCopies();
-    // Return when the bytes have arrived.  `after`: the stream whose work the
+    // Return when the bytes have arrived (page-locked host memory by the driver's
+    // copy).  `after`: the stream whose work the
     // copy follows.  Throws Error on a failed copy.
     void to_host(int device, void *host, const void *src, size_t bytes, cudaStream_t after);
     void to_device(int device, void *dst, const void *host, size_t bytes, cudaStream_t after);

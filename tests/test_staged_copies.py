@@ -1,7 +1,7 @@
 """The staged host copies (staging.cu) against a fake CUDA runtime on the CPU:
 every byte arrives in both directions whatever the runtime refuses, the
-page-locked slots, the event, or all but some of the streams.  A refused copy
-itself is an error."""
+page-locked slots, the event, or all but some of the streams.  Host memory that
+is page-locked itself goes without slots.  A refused copy itself is an error."""
 
 from __future__ import annotations
 
@@ -19,6 +19,7 @@ FAKE = r"""
 #include "staging.cuh"
 
 static int g_alloc = 1, g_event = 1, g_copy = 1;
+static cudaMemoryType g_host = cudaMemoryTypeUnregistered;
 static std::atomic<int> g_streams{0};
 static std::atomic<int> g_made{0}, g_plain{0}, g_live{0};
 static char g_stream_tags[64];
@@ -27,6 +28,10 @@ extern "C" {
 const char *cudaGetErrorString(cudaError_t) { return "fake"; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *) {
+    a->type = g_host;
+    return cudaSuccess;
+}
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) {
     if (!g_alloc) return cudaErrorMemoryAllocation;
     *p = std::malloc(n);
@@ -60,8 +65,9 @@ cudaError_t cudaMemcpyAsync(void *to, const void *from, size_t n, cudaMemcpyKind
 }
 
 // 0 and the count of plain copies in *plain, or 1 for an error, 2 for a leak.
-int staged_copy(int alloc, int event, int streams, int copy, int to_host, char *host, char *gpu,
-                size_t bytes, int *plain) {
+int staged_copy(int alloc, int event, int streams, int copy, int locked, int to_host,
+                char *host, char *gpu, size_t bytes, int *plain) {
+    g_host = locked ? cudaMemoryTypeHost : cudaMemoryTypeUnregistered;
     g_alloc = alloc, g_event = event, g_streams = streams, g_copy = copy;
     g_made = 0, g_plain = 0;
     int status = 0;
@@ -92,19 +98,19 @@ def copy(tmp_path_factory):
                     str(csrc / "staging.cu"), str(folder / "fake.cpp"), "-o", str(library),
                     "-lpthread"], check=True)
     function = ctypes.CDLL(str(library)).staged_copy
-    function.argtypes = [ctypes.c_int] * 5 + [ctypes.c_void_p] * 2 + [ctypes.c_size_t,
+    function.argtypes = [ctypes.c_int] * 6 + [ctypes.c_void_p] * 2 + [ctypes.c_size_t,
                                                                       ctypes.c_void_p]
     return function
 
 
-def _run(copy, to_host, size, *, alloc=1, event=1, streams=10, works=1):
+def _run(copy, to_host, size, *, alloc=1, event=1, streams=10, works=1, locked=0):
     rng = np.random.default_rng(size)
     source = rng.integers(0, 256, size, dtype=np.uint8)
     target = np.zeros(size, np.uint8)
     host, gpu = (target, source) if to_host else (source, target)
     plain = ctypes.c_int()
-    status = copy(alloc, event, streams, works, to_host, host.ctypes.data, gpu.ctypes.data, size,
-                  ctypes.byref(plain))
+    status = copy(alloc, event, streams, works, locked, to_host, host.ctypes.data,
+                  gpu.ctypes.data, size, ctypes.byref(plain))
     return status, bool((source == target).all()), plain.value
 
 
@@ -121,6 +127,11 @@ def test_every_byte_arrives(copy, to_host, size):
                                      dict(alloc=0, event=0, streams=0)])
 def test_a_refused_slot_event_or_stream_leaves_the_plain_copy(copy, to_host, refused):
     assert _run(copy, to_host, 3_000_001, **refused) == (0, True, 2)
+
+
+@pytest.mark.parametrize("to_host", [0, 1])
+def test_page_locked_memory_takes_the_plain_copy(copy, to_host):
+    assert _run(copy, to_host, 3_000_001, locked=1) == (0, True, 2)
 
 
 @pytest.mark.parametrize("to_host", [0, 1])
