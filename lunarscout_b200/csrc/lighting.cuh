@@ -13,9 +13,9 @@ struct ls200_vectors {
     float *data = nullptr;  // device [count, 3]
     int count = 0;
     // device [count]: time indices in the order of the vector's longitude
-    // atan2(y, x), to a bin of 0.044 degrees in a long table.  For a polar site the body's local azimuth follows its
-    // longitude, so in this order consecutive steps read neighbouring
-    // horizon bins.
+    // atan2(y, x), to a bin of 0.044 degrees.  For a polar site the body's local
+    // azimuth follows its longitude, so in this order consecutive steps read
+    // neighbouring horizon bins.
     int *order = nullptr;
     int *window = nullptr;  // device [count]: one launch's sub-range of `order`
     float shortest = 0.0f;  // length of the shortest vector (m; 0 with a NaN)

@@ -46,8 +46,9 @@ struct SharedLevels {
 
 // Resident 128-thread blocks per SM the register budget is sized for.  The
 // settled steps (march_near, march_dem_far) issue 55-60 instructions each where
-// the full step took 137, and no pipe is full (FMA 59 %, issue slots 65-73 %):
-// what remains is latency, so the choice is between resident warps and spills.
+// the full step took 137, and nothing is full (ALU pipe 36 %, FMA 35 %, issue
+// slots 71 %): what remains is latency, so the choice is between resident warps
+// and spills.
 // A site-scale tile (4096^2 at 5 m plus regional, 200 km, B200) takes 174.5 ms
 // at 7 (72 registers) and, before the near field had a loop of its own, 183 ms
 // at 7, 185 ms at 8 (64, a few spills), 198 ms at 9 and 218 ms at 10; with the

@@ -17,7 +17,7 @@
 // its own CPU restatement (oracle flag OPT_LADDER) and their distance from
 // the FP64 restatement is measured beside the reference traversal's.  Its far
 // field runs warp-wide with the culls settled by their bounds (march_dem_ladder:
-// eight sites 430 -> 390 ms).
+// eight sites 426 -> 390 ms).
 //
 // Launch configuration (autotuned, never changing results): how the 32 lanes
 // of a job map onto rays (L neighbouring pixels x 32/L adjacent azimuths, L a
@@ -110,7 +110,9 @@ struct WarpLevels {
 // twice where the cell of the footprint's level is not culled, and on a large
 // fine DEM that is every third step.  Two tiles of a 5 m site, ladder_step
 // against full steps: 126 ms / 152 at 2048^2 pixels, 168 / 194 at 4096^2, but
-// 581 / 474 at 6144^2 and 606 / 515 at 8192^2.
+// 581 / 474 at 6144^2 and 606 / 515 at 8192^2.  The rule looks at the largest side
+// of any DEM of the launch: four small sites march in 77 ms beside a regional DEM
+// of 2000^2 pixels (full steps 91), and in 93 beside one of 6000^2 (94).
 constexpr int kFullSteps = 4;
 constexpr int kSettledSide = 4096;  // largest DEM side for ladder_step (pixels)
 

@@ -25,9 +25,9 @@
 // With the same segment inputs the results are bit-identical to the CPU
 // oracle's FP32 restatement under its production mask.
 //
-// The march is bound by instruction issue (its gathers hit L1/L2), so the
-// work per node visit is kept small without changing any rounded value or
-// decision:
+// The march is bound by the latency of a step's chain and by instruction issue
+// (71 % of the slots; its gathers hit L1/L2), so the work per node visit is kept
+// small without changing any rounded value or decision:
 //   * cells come from a sanitized copy of level 0 (invalid -> -32000) packed
 //     with the mips, so validity is one comparison and the four-cell bound
 //     is a plain maximum;
@@ -1297,7 +1297,7 @@ __device__ __forceinline__ float march_dem_tracked(const Table &table, const Dem
 // So a sample needs its slope only when it may raise the maximum, and a step
 // needs the tangent only when its cell is culled: 60 instructions where
 // level0_step takes 200 (a site-scale tile 183 -> 174.5 ms, a preview tile of
-// 20 km rays 265 -> 252 us).  A ray meets a step it does not cover (the DEM's edge,
+// 5 km rays 265 -> 255 us).  A ray meets a step it does not cover (the DEM's edge,
 // an axis-parallel exit) by leaving; the caller's loop goes on from there.
 // Returns the path position reached; every lane of the warp calls it.
 template <bool kCount, class Table, class Tracker>
@@ -1502,10 +1502,10 @@ __device__ __forceinline__ float march_dem_far(const Table &table, const DemView
 // approximate d and the roundings of both sides); otherwise the step is not
 // settled.  (A maximum beyond 1e4, where the reference's slopes end in its
 // 1e-6 m local_x, leaves every bound above it unclear.)  The exit is computed
-// once, for the level reached.  An iteration is bound by its own length and by
-// lanes that differ: 420 instructions with 20 of 32 lanes active, two climbs
-// at 11 lanes among them.  Eight sites 426 -> 390 ms, two of 2048^2 pixels
-// 71.4 -> 62.7 ms, the checkpointing march of one tile 55.5 -> 49.8 ms.
+// once, for the level reached.  It is bound by lanes that differ and by issue:
+// 19.2 of 32 lanes active, 165 instructions a lane's step, 77 % of the slots (four
+// sites of 512^2 to 1500^2 pixels).  Eight sites 426 -> 390 ms, two of 2048^2
+// pixels 71.4 -> 62.7 ms, the checkpointing march of one tile 55.5 -> 49.8 ms.
 struct LadderRay {
     float end;            // s up to which steps may settle (km; -inf: none)
     float observer_z;
