@@ -181,8 +181,9 @@ __device__ __forceinline__ int stage_window(const LightingBatch &B, const Frame3
 // with one) keep several row reads in flight, 16 patches of 125 and 1460 steps of
 // a year 429 and 3055 us against 710 and 4175 with the loops left to the
 // compiler; fractions take 2 and 1, bytes 2 and 2 (1 % better than others, and 4
-// is 7 % worse).
-template <int kSpan, int kDirectUnroll, int kWindowUnroll, class Put>
+// is 7 % worse).  kWindows: launches without groups have no windows at all, nor
+// their shared memory.
+template <int kSpan, bool kWindows, int kDirectUnroll, int kWindowUnroll, class Put>
 __device__ __forceinline__ void exact_samples(const LightingBatch &B, const Frame32 &f,
                                               const float *horizon, int k0, int k1,
                                               bool windowed, float *window, const Put &put) {
@@ -193,9 +194,11 @@ __device__ __forceinline__ void exact_samples(const LightingBatch &B, const Fram
         return t;
     };
     int first = 0, width = 0;
-    if (windowed && k0 < k1) width = stage_window<kSpan>(B, f, horizon, k0, k1, window, first);
-    // One loop for the warp: a lane without a window goes along with the others'.
-    if (!__any_sync(__activemask(), width > 0)) {
+    if (kWindows && windowed && k0 < k1)
+        width = stage_window<kSpan>(B, f, horizon, k0, k1, window, first);
+    // One loop for the warp, the one that most of its lanes want.
+    const unsigned lanes = __activemask();
+    if (!kWindows || 2 * __popc(__ballot_sync(lanes, width > 0)) <= __popc(lanes)) {
 #pragma unroll kDirectUnroll
         for (int k = k0; k < k1; ++k) {
             float azimuth_deg, elevation;
@@ -231,16 +234,17 @@ __device__ __forceinline__ void exact_samples(const LightingBatch &B, const Fram
 // reads 5; 0.75 for the margin, which reads 2).  Four patches, 355 steps of a
 // year and of a day: fractions 461 and 360 us (a window tried in every chunk of
 // 16: 469 and 358; chunks of 10 without windows: 433 and 487), margins 239 and
-// 198 us (366 and 200; a window tried in every chunk of 10: 280 and 205).
+// 186 us (366 and 200; a window tried in every chunk of 10: 280 and 205).  Launches
+// too small for groups take kernels without windows.
 struct ExactSteps {
     int first, last;
     bool windowed;
 };
 
-template <int kSpan>
+template <int kSpan, bool kWindows>
 __device__ __forceinline__ ExactSteps exact_steps(const LightingBatch &B) {
     const int y = blockIdx.y;
-    if (B.group == 0) return ExactSteps{y * B.chunk, min((y + 1) * B.chunk, B.time_count), false};
+    if (!kWindows) return ExactSteps{y * B.chunk, min((y + 1) * B.chunk, B.time_count), false};
     // The first parts of all groups come first: they have the most to do.
     const int groups = gridDim.y / B.group, part = y / groups;
     const int g0 = (y - part * groups) * B.group * B.chunk;
@@ -287,10 +291,12 @@ static int exact_chunks(ls200_context *ctx, LightingBatch &B, int tiles) {
     const int windowed = ordered_chunk(lighting_chunk(ctx, tiles, B.time_count, 16), B.time_count);
     const int chunks = std::max(1, sms * 24 / blocks);
     const int small = std::max(4, (B.time_count + chunks - 1) / chunks);
+    if (static_cast<long long>(B.time_count / windowed) * blocks < sms * 8) {
+        B.chunk = std::min(small, windowed);
+        return (B.time_count + B.chunk - 1) / B.chunk;
+    }
     const int parts = std::max(1, (windowed + small - 1) / small);
     B.chunk = (windowed + parts - 1) / parts;
-    if (static_cast<long long>(B.time_count / windowed) * blocks < sms * 8)
-        return (B.time_count + B.chunk - 1) / B.chunk;
     B.group = parts;
     const int steps = parts * B.chunk;
     return (B.time_count + steps - 1) / steps * parts;
@@ -686,13 +692,13 @@ __global__ void __launch_bounds__(128, kStagedBlocks)
 }
 
 // Margins, and fractions of launches that are not staged: every sample exactly.
-template <int kSpan, class T>
+template <int kSpan, class T, bool kWindows>
 __global__ void __launch_bounds__(128) lighting_kernel(const __grid_constant__ LightingBatch B) {
-    __shared__ float windows[128 * kWindowStride];
+    __shared__ float windows[kWindows ? 128 * kWindowStride : 1];
     const int tile = blockIdx.z;
     const int index = blockIdx.x * 128 + threadIdx.x;
     const TileGeo &g = B.tiles[tile];
-    const ExactSteps steps = exact_steps<kSpan>(B);
+    const ExactSteps steps = exact_steps<kSpan, kWindows>(B);
     const StoreSample<T> op{static_cast<T *>(B.out) +
                                 static_cast<size_t>(tile) * B.time_count * (kPatch * kPatch) +
                                 index,
@@ -703,9 +709,9 @@ __global__ void __launch_bounds__(128) lighting_kernel(const __grid_constant__ L
         return;
     }
     const size_t pixel = static_cast<size_t>(tile) * kPatch * kPatch + index;
-    exact_samples<kSpan, kSpan == 2 ? 3 : 2, kSpan == 2 ? 4 : sizeof(T) == 1 ? 2 : 1>(
+    exact_samples<kSpan, kWindows, kSpan == 2 ? 3 : 2, kSpan == 2 ? 4 : sizeof(T) == 1 ? 2 : 1>(
         B, load_frame(B.frames, pixel), B.horizons + pixel * kAzimuths, steps.first, steps.last,
-        steps.windowed, windows + threadIdx.x * kWindowStride,
+        steps.windowed, windows + (kWindows ? threadIdx.x * kWindowStride : 0),
         [&](int t, float signal) { op.step(t, signal); });
 }
 
@@ -929,12 +935,15 @@ void lighting_launch(ls200_context *ctx, LightingBatch &B, int tiles, int signal
             staged_fraction_kernel<float><<<grid, 128, 0, ctx->stream>>>(B);
     } else {
         dim3 grid(kPatch * kPatch / 128, exact_chunks(ctx, B, tiles), tiles);
-        if (signal == kSignalFraction)
-            lighting_kernel<5, float><<<grid, 128, 0, ctx->stream>>>(B);
-        else if (signal == kSignalBytes)
-            lighting_kernel<5, uint8_t><<<grid, 128, 0, ctx->stream>>>(B);
-        else
-            lighting_kernel<2, float><<<grid, 128, 0, ctx->stream>>>(B);
+        const auto kernel = signal == kSignalFraction
+                                ? (B.group ? lighting_kernel<5, float, true>
+                                           : lighting_kernel<5, float, false>)
+                            : signal == kSignalBytes
+                                ? (B.group ? lighting_kernel<5, uint8_t, true>
+                                           : lighting_kernel<5, uint8_t, false>)
+                                : (B.group ? lighting_kernel<2, float, true>
+                                           : lighting_kernel<2, float, false>);
+        kernel<<<grid, 128, 0, ctx->stream>>>(B);
     }
     LS_CUDA(cudaGetLastError());
 }
@@ -1027,11 +1036,11 @@ __global__ void __launch_bounds__(128, kStagedBlocks)
 }
 
 // The same without an order, or for a short table: every sample exactly.
-template <int kSpan, bool kAtLeast>
+template <int kSpan, bool kAtLeast, bool kWindows>
 __global__ void __launch_bounds__(128) signal_bits_kernel(const __grid_constant__ LightingBatch B,
                                                           float threshold, int words,
                                                           uint32_t *__restrict__ bits) {
-    __shared__ float windows[128 * kWindowStride];
+    __shared__ float windows[kWindows ? 128 * kWindowStride : 1];
     const int index = blockIdx.x * 128 + threadIdx.x;
     const TileGeo &g = B.tiles[blockIdx.z];
     if (index % kPatch >= g.valid_width || index / kPatch >= g.valid_height) return;
@@ -1039,10 +1048,10 @@ __global__ void __launch_bounds__(128) signal_bits_kernel(const __grid_constant_
     const SetBit<kSpan, kAtLeast> op{
         bits + static_cast<size_t>(blockIdx.z) * words * (kPatch * kPatch) + index, threshold,
         false, false};
-    const ExactSteps steps = exact_steps<kSpan>(B);
-    exact_samples<kSpan, kSpan == 2 ? 3 : 1, kSpan == 2 ? 4 : 1>(
+    const ExactSteps steps = exact_steps<kSpan, kWindows>(B);
+    exact_samples<kSpan, kWindows, kSpan == 2 ? 3 : 1, kSpan == 2 ? 4 : 1>(
         B, load_frame(B.frames, pixel), B.horizons + pixel * kAzimuths, steps.first, steps.last,
-        steps.windowed, windows + threadIdx.x * kWindowStride,
+        steps.windowed, windows + (kWindows ? threadIdx.x * kWindowStride : 0),
         [&](int t, float signal) { op.step(t, signal); });
 }
 
@@ -1065,8 +1074,11 @@ static void signal_bits_launch(ls200_context *ctx, LightingBatch B, int tiles,
     if (staged)
         staged_bits_kernel<kSpan, kAtLeast>
             <<<grid, 128, 0, ctx->stream>>>(B, threshold, words, bits);
+    else if (B.group)
+        signal_bits_kernel<kSpan, kAtLeast, true>
+            <<<grid, 128, 0, ctx->stream>>>(B, threshold, words, bits);
     else
-        signal_bits_kernel<kSpan, kAtLeast>
+        signal_bits_kernel<kSpan, kAtLeast, false>
             <<<grid, 128, 0, ctx->stream>>>(B, threshold, words, bits);
     LS_CUDA(cudaGetLastError());
 }
@@ -1435,19 +1447,21 @@ __global__ void __launch_bounds__(128, kStagedBlocks)
 }
 
 // The same without an order, or for a short table: every sample exactly.
+template <bool kWindows>
 __global__ void __launch_bounds__(128) visibility_kernel(const __grid_constant__ LightingBatch B,
                                                          float threshold,
                                                          unsigned *__restrict__ counts) {
-    __shared__ float windows[128 * kWindowStride];
+    __shared__ float windows[kWindows ? 128 * kWindowStride : 1];
     const int index = blockIdx.x * 128 + threadIdx.x;
     const TileGeo &g = B.tiles[blockIdx.z];
     if (index % kPatch >= g.valid_width || index / kPatch >= g.valid_height) return;
     const size_t pixel = static_cast<size_t>(blockIdx.z) * kPatch * kPatch + index;
     CountVisible op{counts + pixel, threshold, 0u};
-    const ExactSteps steps = exact_steps<2>(B);
-    exact_samples<2, 3, 4>(B, load_frame(B.frames, pixel), B.horizons + pixel * kAzimuths, steps.first,
-                     steps.last, steps.windowed, windows + threadIdx.x * kWindowStride,
-                     [&](int t, float signal) { op.step(t, signal); });
+    const ExactSteps steps = exact_steps<2, kWindows>(B);
+    exact_samples<2, kWindows, 3, 4>(
+        B, load_frame(B.frames, pixel), B.horizons + pixel * kAzimuths, steps.first, steps.last,
+        steps.windowed, windows + (kWindows ? threadIdx.x * kWindowStride : 0),
+        [&](int t, float signal) { op.step(t, signal); });
     if (op.count) atomicAdd(op.counts, op.count);
 }
 
@@ -1478,8 +1492,10 @@ void visibility_launch(ls200_context *ctx, LightingBatch &B, int tiles,
               staged ? staged_chunks(B) : exact_chunks(ctx, B, tiles), tiles);
     if (staged)
         staged_visibility_kernel<<<grid, 128, 0, ctx->stream>>>(B, threshold, counts);
+    else if (B.group)
+        visibility_kernel<true><<<grid, 128, 0, ctx->stream>>>(B, threshold, counts);
     else
-        visibility_kernel<<<grid, 128, 0, ctx->stream>>>(B, threshold, counts);
+        visibility_kernel<false><<<grid, 128, 0, ctx->stream>>>(B, threshold, counts);
     LS_CUDA(cudaGetLastError());
     visibility_finalize<<<(n + 255) / 256, 256, 0, ctx->stream>>>(counts, n, B.time_count, valid,
                                                                   out);
