@@ -674,7 +674,7 @@ struct StoreSample {
 constexpr int kStagedBlocks = 7;
 
 // Sun fractions of an ordered launch.  Four patches, 8761 steps, bytes (B200,
-// whole call): 5.66 ms with the exact functions for every sample, 2.08 ms.  A
+// whole call): 5.66 ms with the exact functions for every sample, 1.89 ms.  A
 // warp's step takes 48 instructions with its share of exact samples (about 14),
 // a chunk's staging 2300; 78 % of the issue slots are busy.
 template <class T>
